@@ -115,31 +115,6 @@ __device__ __forceinline__ TileInfo decode_tile(const TcProblem &p, long t) {
   return ti;
 }
 
-// split 8 floats into hi / mid / lo BF16 (packed pairs, element 0 in the low half)
-template <int NSPLIT>
-__device__ __forceinline__ void split8(const float *x, uint4 &h, uint4 &m, uint4 &l) {
-  uint32_t hh[4], mm[4], ll[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float x0 = x[2 * i], x1 = x[2 * i + 1];
-    __nv_bfloat162 b = __floats2bfloat162_rn(x0, x1);
-    const float r0 = x0 - __low2float(b), r1 = x1 - __high2float(b);
-    __nv_bfloat162 c = __floats2bfloat162_rn(r0, r1);
-    hh[i] = *reinterpret_cast<uint32_t *>(&b);
-    mm[i] = *reinterpret_cast<uint32_t *>(&c);
-    if (NSPLIT == 3) {
-      const float s0 = r0 - __low2float(c), s1 = r1 - __high2float(c);
-      __nv_bfloat162 d = __floats2bfloat162_rn(s0, s1);
-      ll[i] = *reinterpret_cast<uint32_t *>(&d);
-    } else {
-      ll[i] = 0;
-    }
-  }
-  h = make_uint4(hh[0], hh[1], hh[2], hh[3]);
-  m = make_uint4(mm[0], mm[1], mm[2], mm[3]);
-  l = make_uint4(ll[0], ll[1], ll[2], ll[3]);
-}
-
 // ---- cp.async (global -> shared), zero fill past src_bytes ----
 __device__ __forceinline__ void cp_async16(uint32_t saddr, const void *g, int src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(saddr), "l"(g),
@@ -612,23 +587,6 @@ struct WsArgs {
   int c_tma;          // C written by TMA stores (boxes of 32 columns x 32 rows)
 };
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(ptx::smem_u32(bar)) : "memory");
-}
-// Arrival that publishes no memory.  The default arrive has release
-// semantics: it orders this thread's earlier memory operations, the
-// epilogue's global C stores included, before the arrival.  Arrivals that
-// only say "done reading" (TMEM read back and waited for, a queue slot
-// copied into registers) have nothing to publish.
-__device__ __forceinline__ void mbar_arrive_relaxed(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.relaxed.cta.shared::cta.b64 _, [%0];" ::"r"(ptx::smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;" ::"r"(bytes),
-               "r"(ptx::smem_u32(bar))
-               : "memory");
-}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint64_t *bar,
                                             int c0, int c1, int c2) {
   asm volatile(
@@ -636,36 +594,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
       " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(ptx::smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
-}
-
-// Slow path of ws_wait: the thread suspends in the barrier wait (up to about
-// a microsecond per try, woken when the phase completes) instead of polling,
-// so waiting roles take no issue slots or shared-memory bandwidth from the
-// working ones.  Gives up after `limit` tries or two seconds, whichever
-// comes first, or as soon as another role has aborted.  Inlined: a call
-// would make the caller save its live registers to local memory around every
-// wait.
-__device__ __forceinline__ bool ws_wait_slow(uint64_t *bar, uint32_t parity,
-                                             volatile int *abort_flag, unsigned *err,
-                                             uint32_t limit) {
-  const uint64_t t0 = ptx::globaltimer_ns();
-  for (uint32_t it = 0; it < limit; ++it) {
-    if (ptx::mbar_try_wait_suspend(bar, parity, 1000)) return true;
-    if ((it & 15) == 15) {
-      if (*abort_flag) return false;
-      if (ptx::globaltimer_ns() - t0 > 2000000000ull) break;
-    }
-  }
-  *abort_flag = 1;
-  atomicOr(err, 1u);
-  return false;
-}
-
-// Bounded wait: one test inline, the rest in ws_wait_slow.
-__device__ __forceinline__ bool ws_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag,
-                                        unsigned *err, uint32_t limit = 1u << 22) {
-  if (ptx::mbar_try_wait(bar, parity)) return true;
-  return ws_wait_slow(bar, parity, abort_flag, err, limit);
 }
 
 // BLX > 0: each epilogue warp holds at most BLX 32-column blocks of C (a
@@ -736,28 +664,24 @@ __global__ void __launch_bounds__(WsRoles<WIDE>::THREADS, 1)
     }
   } else if (warp == 1) {
     // -------------------------------- MMA ---------------------------------
-    if (lane == 0) {
-      const uint32_t idesc = ptx::idesc_bf16_f32(TC_BM, tn);
-      long j = 0, u = 0;
-      bool ok = true;
-      for (long t = blockIdx.x; ok && t < p.num_tiles; t += gridDim.x) {
-        for (int s = 0; ok && s < p.nk; ++s, ++j) {
-          const int s_in = s % kc;
-          if (s_in == 0) {
-            // new accumulation chunk: wait until the epilogue has drained this set
-            const int a = (int)(u & 1);
-            if (u >= 2 && !ws_wait(&bars[B_AEMPTY + a], (uint32_t)(((u >> 1) - 1) & 1), s_abort,
-                                   p.err)) {
-              ok = false;
-              break;
-            }
-          }
-          const int b = (int)(j & 1);
-          if (!ws_wait(&bars[B_BFULL + b], (uint32_t)((j >> 1) & 1), s_abort, p.err)) {
-            ok = false;
-            break;
-          }
-          ptx::tc_fence_after();
+    // the whole warp waits, one elected lane issues
+    const unsigned FULL = 0xffffffffu;
+    const uint32_t idesc = ptx::idesc_bf16_f32(TC_BM, tn);
+    long j = 0, u = 0;
+    bool ok = true;
+    for (long t = blockIdx.x; ok && t < p.num_tiles; t += gridDim.x) {
+      for (int s = 0; s < p.nk; ++s, ++j) {
+        const int s_in = s % kc;
+        // new accumulation chunk: wait until the epilogue has drained this set
+        if (s_in == 0 && u >= 2)
+          ok = ws_wait(&bars[B_AEMPTY + (u & 1)], (uint32_t)(((u >> 1) - 1) & 1), s_abort, p.err);
+        const int b = (int)(j & 1);
+        if (ok) ok = ws_wait(&bars[B_BFULL + b], (uint32_t)((j >> 1) & 1), s_abort, p.err);
+        ok = __all_sync(FULL, ok);
+        if (!ok) break;
+        ptx::tc_fence_after();
+        const bool last = s_in == kc - 1 || s == p.nk - 1;
+        if (ptx::elect_one()) {
           const uint32_t acc_base = tmem + (uint32_t)((u & 1) * 256);
           const uint32_t bb = smem_base + WS_OFF_BUF + b * BUF_BYTES;
           const int ksteps = min(2, (p.K - s * TC_BK + 15) / 16);
@@ -782,16 +706,16 @@ __global__ void __launch_bounds__(WsRoles<WIDE>::THREADS, 1)
             }
           }
           ptx::mma_commit(&bars[B_BEMPTY + b]);  // operand buffer b may be refilled
-          if (s_in == kc - 1 || s == p.nk - 1) {
-            ptx::mma_commit(&bars[B_AFULL + (u & 1)]);  // accumulation chunk complete
-            ++u;
-          }
+          if (last) ptx::mma_commit(&bars[B_AFULL + (u & 1)]);  // accumulation chunk complete
         }
+        __syncwarp();
+        if (last) ++u;
       }
-      // every MMA this thread issued has completed before TMEM is freed
-      ptx::mma_commit(&bars[B_FINAL]);
-      ptx::mbar_wait_bounded(&bars[B_FINAL], 0);
     }
+    // every MMA issued has completed before TMEM is freed
+    if (ptx::elect_one()) ptx::mma_commit(&bars[B_FINAL]);
+    __syncwarp();
+    ptx::mbar_wait_bounded(&bars[B_FINAL], 0);
   } else if (warp < Roles::W_EPI) {
     // ----------------------------- converters -----------------------------
     // items of a slab: A (row cr, 8-k chunk c) and B (column jj, chunk c),
@@ -1253,12 +1177,6 @@ __device__ __forceinline__ bool q_get(const unsigned char *smem, long j, GItem &
   return true;
 }
 
-// C[i] += v at L2 (red.global.add.f32: round to nearest even; subnormal
-// inputs and sums flush to zero)
-__device__ __forceinline__ void red_add_f32(float *p, float v) {
-  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
-}
-
 __device__ __forceinline__ void cp_async_mbar_arrive(uint64_t *bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(ptx::smem_u32(bar))
                : "memory");
@@ -1419,8 +1337,9 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_tc_grouped(const GrpArgs g) {
   } else if (warp == G_W_MMA) {
     // -------------------------------- MMA ---------------------------------
     // The whole warp walks the items and waits, so that none of its lanes
-    // sits at the block barrier while the issuing lane works; lane 0 issues
-    // the MMAs and the commits.
+    // sits at the block barrier while the issuing lane works; one elected
+    // lane issues the MMAs and the commits (the same one every time: commits
+    // cover the MMAs of the thread that issues them).
     const unsigned FULL = 0xffffffffu;
     long js = 0, u = 0;
     bool ok = true;
@@ -1450,7 +1369,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_tc_grouped(const GrpArgs g) {
         }
         ptx::tc_fence_after();
         const bool last = s_in == kc - 1 || s == it.nk - 1;
-        if (lane == 0) {
+        if (ptx::elect_one()) {
           const uint32_t acc_base = tmem + (uint32_t)((u & 1) * 256);
           const uint32_t bb = smem_base + WS_OFF_BUF + b * BUF_BYTES;
           const int ksteps = max(1, min(2, (it.K - s * TC_BK + 15) / 16));
@@ -1481,7 +1400,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_tc_grouped(const GrpArgs g) {
         if (last) ++u;
       }
     }
-    if (lane == 0) ptx::mma_commit(&bars[B_FINAL]);
+    if (ptx::elect_one()) ptx::mma_commit(&bars[B_FINAL]);
     __syncwarp();
     ptx::mbar_wait_bounded(&bars[B_FINAL], 0);
   } else if (warp < G_W_EPI0) {

@@ -3,6 +3,7 @@
 // the shared-memory / instruction descriptors the MMA consumes.
 #pragma once
 
+#include <cuda_bf16.h>
 #include <stdint.h>
 
 namespace ls {
@@ -128,6 +129,18 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
       : "memory");
 }
 
+// True in one lane of a converged warp.  MMAs issued under this predicate
+// keep their descriptors in uniform registers: a burst of 12 MMAs of
+// 128 x 32 x 16 takes 471 cycles to issue instead of 658 under `lane == 0`
+// (64 x 32 x 16: 311 instead of 658).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+
 // Arrives (once) on the mbarrier when all tcgen05 ops issued so far by this
 // thread have completed.
 __device__ __forceinline__ void mma_commit(uint64_t *bar) {
@@ -190,4 +203,110 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n) {
 }
 
 }  // namespace ptx
+
+// ---- hand-offs shared by the tensor-core kernels -------------------------------
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(ptx::smem_u32(bar)) : "memory");
+}
+// Arrival that publishes no memory.  The default arrive has release
+// semantics: it orders this thread's earlier memory operations, the
+// epilogue's global C stores included, before the arrival.  Arrivals that
+// only say "done reading" (TMEM read back and waited for, a queue slot
+// copied into registers) have nothing to publish.
+__device__ __forceinline__ void mbar_arrive_relaxed(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.relaxed.cta.shared::cta.b64 _, [%0];" ::"r"(ptx::smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_tx(uint64_t *bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;" ::"r"(bytes),
+               "r"(ptx::smem_u32(bar))
+               : "memory");
+}
+// Slow path of ws_wait: the thread suspends in the barrier wait (up to about
+// a microsecond per try, woken when the phase completes) instead of polling,
+// so waiting roles take no issue slots or shared-memory bandwidth from the
+// working ones.  Gives up after `limit` tries or two seconds, whichever
+// comes first, or as soon as another role has aborted.  Inlined: a call
+// would make the caller save its live registers to local memory around every
+// wait.
+__device__ __forceinline__ bool ws_wait_slow(uint64_t *bar, uint32_t parity,
+                                             volatile int *abort_flag, unsigned *err,
+                                             uint32_t limit) {
+  const uint64_t t0 = ptx::globaltimer_ns();
+  for (uint32_t it = 0; it < limit; ++it) {
+    if (ptx::mbar_try_wait_suspend(bar, parity, 1000)) return true;
+    if ((it & 15) == 15) {
+      if (*abort_flag) return false;
+      if (ptx::globaltimer_ns() - t0 > 2000000000ull) break;
+    }
+  }
+  *abort_flag = 1;
+  atomicOr(err, 1u);
+  return false;
+}
+
+// Bounded wait: one test inline, the rest in ws_wait_slow.
+__device__ __forceinline__ bool ws_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag,
+                                        unsigned *err, uint32_t limit = 1u << 22) {
+  if (ptx::mbar_try_wait(bar, parity)) return true;
+  return ws_wait_slow(bar, parity, abort_flag, err, limit);
+}
+
+// C[i] += v at L2 (red.global.add.f32: round to nearest even; subnormal
+// inputs and sums flush to zero)
+__device__ __forceinline__ void red_add_f32(float *p, float v) {
+  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+
+// two floats in one 64-bit register, and the packed FP32 operations on them
+// (each half rounded like the scalar operation)
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// The split is the busiest step of these kernels' issue slots: the packed
+// FMA takes the two subtractions of a pair at once.  x - float(b), both
+// halves (exact: b is x rounded to BF16)
+__device__ __forceinline__ uint64_t bf16_rest(uint64_t x, uint32_t b) {
+  const uint64_t f = (uint64_t)(b & 0xffff0000u) << 32 | (uint64_t)(b << 16);
+  return fma2(f, 0xbf800000bf800000ull, x);  // f * -1 + x
+}
+__device__ __forceinline__ uint32_t bf16_round(uint64_t x) {
+  float lo, hi;
+  unpack2(x, lo, hi);
+  __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<uint32_t *>(&b);
+}
+
+// split 8 floats into hi / mid / lo BF16 (packed pairs, element 0 in the low half)
+template <int NSPLIT>
+__device__ __forceinline__ void split8(const float *x, uint4 &h, uint4 &m, uint4 &l) {
+  uint32_t hh[4], mm[4], ll[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint64_t x2 = pack2(x[2 * i], x[2 * i + 1]);
+    hh[i] = bf16_round(x2);
+    const uint64_t r2 = bf16_rest(x2, hh[i]);
+    mm[i] = bf16_round(r2);
+    ll[i] = NSPLIT == 3 ? bf16_round(bf16_rest(r2, mm[i])) : 0u;
+  }
+  h = make_uint4(hh[0], hh[1], hh[2], hh[3]);
+  m = make_uint4(mm[0], mm[1], mm[2], mm[3]);
+  l = make_uint4(ll[0], ll[1], ll[2], ll[3]);
+}
+
 }  // namespace ls
