@@ -1038,15 +1038,34 @@ __global__ void __launch_bounds__(WsRoles<WIDE>::THREADS, 1)
 // ===========================================================================
 constexpr int GRP_CLASSES = 64;  // work classes (total K slabs of the run, capped)
 
+// Plan of a grouped batch.  Runs whose C is at most 256 x 256 become one item
+// per tile of the small-product kernel; larger runs go to k_tc_grouped, one
+// item per run.  Runs of full tiles with 16-byte aligned operands can go to
+// either: k_tc_grouped is faster on them (128 x 128 x 512 NT, 1,500 products:
+// 352 against 502 us; 256^3 NT, 1,000: 463 against 584 us), but as a second
+// kernel it only pays when there are enough of them to fill the machine.
+enum : int { GRP_SMALL = 0, GRP_LARGE = 1, GRP_EITHER = 2, GRP_EMPTY = 3 };
+constexpr int GRP_SMALL_EDGE = 256;
+constexpr int GRP_SMALL_TILES =
+    (GRP_SMALL_EDGE / SM_SMALL_TM) * (GRP_SMALL_EDGE / SM_SMALL_TN);
+constexpr long GRP_SMALL_MAX_COUNT = 1L << 24;  // 1 GB of items
+static_assert(GRP_SMALL_TILES <= 8, "an item word holds three bits of tile");
+
 // workspace layout of the plan (unsigned words)
 struct GrpPlan {
-  unsigned *class_runs;   // [GRP_CLASSES] runs per class
-  unsigned *class_off;    // [GRP_CLASSES] first sorted slot of each class
-  unsigned *class_fill;   // [GRP_CLASSES] slots taken so far
-  unsigned *n_runs;       // [1]
-  unsigned *run_first;    // [count] first entry of the run in sorted slot s
-  unsigned *run_len;      // [count]
+  unsigned *class_n;     // [4][GRP_CLASSES] per class: items of the small runs, the large
+                         // runs, items of the runs that can be either, those runs
+  unsigned *class_off;   // [2][GRP_CLASSES] first sorted slot of each class (small, large)
+  unsigned *class_fill;  // [2][GRP_CLASSES] slots taken so far
+  unsigned *n_items;     // [2] items of the small-product kernel, runs of k_tc_grouped
+  unsigned *counter;     // [1] work counter of the small-product kernel
+  unsigned *either_large;  // [1] where the runs that can be either go
+  unsigned either_min;     // runs that can be either for them to go to k_tc_grouped
+  uint2 *items;          // [GRP_SMALL_TILES * count]; null: every run is large
+  unsigned *run_first;   // [count] first entry of the large run in sorted slot s
+  unsigned *run_len;     // [count]
 };
+constexpr int GRP_HEADER = 1024;  // words of the class tables and counts
 
 struct GrpArgs {
   const LibShalom_sgemm_entry *entries;
@@ -1063,50 +1082,101 @@ __device__ __forceinline__ bool grp_run_start(const LibShalom_sgemm_entry *e, lo
   return i == 0 || e[i].C != e[i - 1].C;
 }
 
-// K work of the run starting at entry i (capped class index) and its length
+// The run starting at entry i: K work (capped class index), length, kernel
+// and tiles in the small-product kernel
 __device__ __forceinline__ int grp_run_class(const LibShalom_sgemm_entry *e, long count, long i,
-                                             long *len) {
+                                             bool with_small, long *len, int *kind, int *tiles) {
+  const int M = e[i].M, N = e[i].N;
+  // share of the 128 x 128 tiles that C fills, at least 85 %
+  const bool full = (long)M * N * 20 >= 17L * ((M + 127) / 128) * ((N + 127) / 128) * 16384;
+  bool fits = M <= GRP_SMALL_EDGE && N <= GRP_SMALL_EDGE, either = true;
   long slabs = 0, j = i;
   do {
-    slabs += max(1, (e[j].K + TC_BK - 1) / TC_BK);
+    const LibShalom_sgemm_entry &x = e[j];
+    slabs += max(1, (x.K + TC_BK - 1) / TC_BK);
+    fits = fits && max(x.K, max(x.lda, x.ldb)) < (1 << 30);
+    const int lda = x.lda > 0 ? x.lda : x.K, ldb = x.ldb > 0 ? x.ldb : x.transb ? x.K : N;
+    either = either && (((uintptr_t)x.A | (uintptr_t)x.B) & 15) == 0 && ((lda | ldb) & 3) == 0 &&
+             ((x.transb && x.K >= 128 && full) || (x.K > 256 && M >= 128));
     ++j;
   } while (j < count && e[j].C == e[i].C);
   *len = j - i;
+  *tiles = ((M + SM_SMALL_TM - 1) / SM_SMALL_TM) * ((N + SM_SMALL_TN - 1) / SM_SMALL_TN);
+  *kind = M <= 0 || N <= 0                                ? GRP_EMPTY
+          : !with_small || !fits || j - i >= (1L << 28) ? GRP_LARGE
+          : either                                        ? GRP_EITHER
+                                                          : GRP_SMALL;
   return (int)min(slabs, (long)GRP_CLASSES - 1);
 }
 
-// pass 1: runs per work class
+// pass 1: items per work class
 __global__ void k_grp_count(const LibShalom_sgemm_entry *e, long count, GrpPlan pl) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count;
        i += (long)gridDim.x * blockDim.x) {
     if (!grp_run_start(e, i)) continue;
     long len;
-    atomicAdd(&pl.class_runs[grp_run_class(e, count, i, &len)], 1u);
-  }
-}
-
-// pass 2: first sorted slot of every class, heaviest class first
-__global__ void k_grp_offsets(GrpPlan pl) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    unsigned acc = 0;
-    for (int c = GRP_CLASSES - 1; c >= 0; --c) {
-      pl.class_off[c] = acc;
-      acc += pl.class_runs[c];
+    int kind, tiles;
+    const int cls = grp_run_class(e, count, i, pl.items != nullptr, &len, &kind, &tiles);
+    if (kind == GRP_SMALL) atomicAdd(&pl.class_n[cls], (unsigned)tiles);
+    if (kind == GRP_LARGE) atomicAdd(&pl.class_n[GRP_CLASSES + cls], 1u);
+    if (kind == GRP_EITHER) {
+      atomicAdd(&pl.class_n[2 * GRP_CLASSES + cls], (unsigned)tiles);
+      atomicAdd(&pl.class_n[3 * GRP_CLASSES + cls], 1u);
     }
-    *pl.n_runs = acc;
   }
 }
 
-// pass 3: every run takes a slot in its class's range
+// pass 2: first sorted slot of every class, heaviest class first (one block of
+// GRP_CLASSES threads)
+__global__ void __launch_bounds__(GRP_CLASSES) k_grp_offsets(GrpPlan pl) {
+  __shared__ unsigned n[4][GRP_CLASSES];
+  __shared__ int s_large;
+  const int c = threadIdx.x;
+  for (int k = 0; k < 4; ++k) n[k][c] = pl.class_n[k * GRP_CLASSES + c];
+  __syncthreads();
+  if (c == 0) {
+    unsigned runs = 0;
+    for (int i = 0; i < GRP_CLASSES; ++i) runs += n[3][i];
+    s_large = runs >= pl.either_min;
+    *pl.either_large = s_large;
+  }
+  __syncthreads();
+  unsigned before[2] = {0, 0};
+  for (int i = GRP_CLASSES - 1; i >= c; --i) {
+    const unsigned s = n[0][i] + (s_large ? 0u : n[2][i]), l = n[1][i] + (s_large ? n[3][i] : 0u);
+    if (i > c) {
+      before[0] += s;
+      before[1] += l;
+    } else if (c == 0) {
+      pl.n_items[0] = before[0] + s;
+      pl.n_items[1] = before[1] + l;
+    }
+  }
+  pl.class_off[c] = before[0];
+  pl.class_off[GRP_CLASSES + c] = before[1];
+}
+
+// pass 3: every item takes a slot in its class's range
 __global__ void k_grp_place(const LibShalom_sgemm_entry *e, long count, GrpPlan pl) {
+  const bool either_large = *pl.either_large != 0;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count;
        i += (long)gridDim.x * blockDim.x) {
     if (!grp_run_start(e, i)) continue;
     long len;
-    const int cls = grp_run_class(e, count, i, &len);
-    const unsigned slot = pl.class_off[cls] + atomicAdd(&pl.class_fill[cls], 1u);
-    pl.run_first[slot] = (unsigned)i;
-    pl.run_len[slot] = (unsigned)len;
+    int kind, tiles;
+    int cls = grp_run_class(e, count, i, pl.items != nullptr, &len, &kind, &tiles);
+    if (kind == GRP_EMPTY) continue;
+    const bool large = kind == GRP_LARGE || (kind == GRP_EITHER && either_large);
+    if (large) cls += GRP_CLASSES;
+    const unsigned slot =
+        pl.class_off[cls] + atomicAdd(&pl.class_fill[cls], large ? 1u : (unsigned)tiles);
+    if (large) {
+      pl.run_first[slot] = (unsigned)i;
+      pl.run_len[slot] = (unsigned)len;
+    } else {
+      for (int t = 0; t < tiles; ++t)
+        pl.items[slot + t] = make_uint2((unsigned)i, (unsigned)len << 3 | (unsigned)t);
+    }
   }
 }
 
@@ -1227,6 +1297,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_tc_grouped(const GrpArgs g) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t smem_base = ptx::smem_u32(smem);
   const int kc = g.kc_slabs;
+  if (*g.n_runs == 0) return;  // every run went to the small-product kernel
 
   if (tid == 0) {
     for (int i = 0; i < G_STAGES; ++i) {
@@ -1782,7 +1853,21 @@ int tc_launch(TcProblem &p, int mode) {
   CUtensorMap ma, mb, mc;
   memset(&mc, 0, sizeof(mc));
   WsArgs wa;
-  if (st.use_tma && ws_maps(p, &ma, &mb, &mc, &wa)) {
+  const bool tma = st.use_tma && ws_maps(p, &ma, &mb, &mc, &wa);
+  if (!tma && st.use_tma && !p.kslice && p.lda < (1 << 30) && p.ldb < (1 << 30)) {
+    TcSmallArgs sa{};
+    sa.A = p.A; sa.B = p.B; sa.C = p.C;
+    sa.sA = p.sA; sa.sB = p.sB; sa.sC = p.sC;
+    sa.lda = p.lda; sa.ldb = p.ldb; sa.ldc = p.ldc;
+    sa.M = p.M; sa.N = p.N; sa.K = p.K; sa.transb = p.transb;
+    sa.alpha = p.alpha; sa.beta = p.beta;
+    sa.tiles_n = (int)cdiv(p.N, SM_SMALL_TN);
+    sa.tiles = (int)cdiv(p.M, SM_SMALL_TM) * sa.tiles_n;
+    sa.n_items = (long)sa.tiles * p.count;
+    sa.err = p.err;
+    const int rc = tc_small_launch(sa, true, mode);
+    if (rc) return rc;
+  } else if (tma) {
     const bool wide = !drain && wa.c_tma;
     // long K on tiles of at most 64 columns: one 32-column block per epilogue
     // warp, a fold of 32 registers instead of 64 (no spills)
@@ -1948,35 +2033,55 @@ int tc_sgemm_grouped(const LibShalom_sgemm_entry *entries, long count, int mode)
   if (!tc_mode_ok(mode)) return LIBSHALOM_ERR_INVALID_VALUE;
   if (count > (1L << 30)) return LIBSHALOM_ERR_UNSUPPORTED;
   State &st = state();
-  // plan workspace: 256-word header (class tables, run count), then two
-  // arrays sized by the entry count
-  const size_t words = 256 + 2 * (size_t)count;
+  // plan workspace: a header (class tables, item counts), the large
+  // runs' list and, for batches it is worth the memory for, the items of the
+  // small-product kernel (without them every run counts as large)
+  const size_t words = GRP_HEADER + 2 * (size_t)count;
+  const size_t item_words = 2 * (size_t)GRP_SMALL_TILES * (size_t)count;
   void *ws = nullptr;
-  int rc = workspace(words * sizeof(unsigned), &ws);
-  if (rc) return rc;
+  bool with_small = count <= GRP_SMALL_MAX_COUNT &&
+                    workspace((words + item_words) * sizeof(unsigned), &ws) == LIBSHALOM_SUCCESS;
+  if (!with_small) {
+    const int rc = workspace(words * sizeof(unsigned), &ws);
+    if (rc) return rc;
+  }
   unsigned *w = static_cast<unsigned *>(ws);
   GrpPlan pl;
-  pl.class_runs = w;
-  pl.class_off = w + GRP_CLASSES;
-  pl.class_fill = w + 2 * GRP_CLASSES;
-  pl.n_runs = w + 3 * GRP_CLASSES;
-  pl.run_first = w + 256;
+  pl.class_n = w;
+  pl.class_off = w + 4 * GRP_CLASSES;
+  pl.class_fill = w + 6 * GRP_CLASSES;
+  pl.n_items = w + 8 * GRP_CLASSES;
+  pl.counter = pl.n_items + 2;
+  pl.either_large = pl.n_items + 3;
+  pl.either_min = 2u * (unsigned)st.num_sms;
+  pl.items = with_small ? reinterpret_cast<uint2 *>(w + GRP_HEADER) : nullptr;
+  pl.run_first = w + GRP_HEADER + (with_small ? item_words : 0);
   pl.run_len = pl.run_first + count;
-  LS_CUDA_TRY(cudaMemsetAsync(w, 0, 256 * sizeof(unsigned), st.stream));
+  LS_CUDA_TRY(cudaMemsetAsync(w, 0, GRP_HEADER * sizeof(unsigned), st.stream));
   const int pgrid = (int)std::max(1L, std::min(cdiv(count, 256), (long)st.num_sms * 8));
   k_grp_count<<<pgrid, 256, 0, st.stream>>>(entries, count, pl);
-  k_grp_offsets<<<1, 32, 0, st.stream>>>(pl);
+  k_grp_offsets<<<1, GRP_CLASSES, 0, st.stream>>>(pl);
   k_grp_place<<<pgrid, 256, 0, st.stream>>>(entries, count, pl);
   LS_CUDA_TRY(cudaGetLastError());
 
   void *errp = nullptr;
   LS_CUDA_TRY(cudaGetSymbolAddress(&errp, g_tc_err));
+  if (with_small) {
+    TcSmallArgs sa{};
+    sa.entries = entries;
+    sa.items = pl.items;
+    sa.n_items_dev = pl.n_items;
+    sa.counter = pl.counter;
+    sa.err = reinterpret_cast<unsigned *>(errp);
+    const int rc = tc_small_launch(sa, false, mode);
+    if (rc) return rc;
+  }
   GrpArgs g;
   g.entries = entries;
   g.count = count;
   g.run_first = pl.run_first;
   g.run_len = pl.run_len;
-  g.n_runs = pl.n_runs;
+  g.n_runs = pl.n_items + 1;
   g.err = reinterpret_cast<unsigned *>(errp);
   g.kc_slabs = 128 / TC_BK;
   const void *kern = mode == LIBSHALOM_PREC_BF16X6 ? (const void *)k_tc_grouped<3>

@@ -18,6 +18,26 @@ int tc_sgemm_strided(const GemmArgs<float> &g, long sA, long sB, long sC, long c
 // Grouped batch (entries in device memory) on the tensor cores.
 int tc_sgemm_grouped(const LibShalom_sgemm_entry *entries, long count, int mode);
 
+// Tiles of the small-product kernel (ls_tc_small.cu): C rows and columns.
+constexpr int SM_SMALL_TM = 64, SM_SMALL_TN = 128;
+
+// Work of the small-product kernel.  Grouped: items {first entry of the run,
+// products << 3 | tile} in device memory.  Uniform: GEMM g of the batch at
+// A + g * sA etc., `tiles` tiles each.
+struct TcSmallArgs {
+  const LibShalom_sgemm_entry *entries;
+  const uint2 *items;
+  const unsigned *n_items_dev;
+  unsigned *counter;  // zeroed before the launch
+  const float *A, *B;
+  float *C;
+  long sA, sB, sC, lda, ldb, ldc, n_items;
+  int M, N, K, transb, tiles, tiles_n;
+  float alpha, beta;
+  unsigned *err;  // device status word (bounded waits)
+};
+int tc_small_launch(const TcSmallArgs &a, bool uniform, int mode);
+
 // Runs the bounded-wait self-check kernel (an mbarrier nothing arrives at);
 // returns LIBSHALOM_ERR_DEVICE_TIMEOUT when its waits expired and reported.
 int tc_wait_expiry_selftest(int iterations);

@@ -309,4 +309,34 @@ __device__ __forceinline__ void split8(const float *x, uint4 &h, uint4 &m, uint4
   l = make_uint4(ll[0], ll[1], ll[2], ll[3]);
 }
 
+// predicated global accesses (a predicate, not a branch, per access)
+__device__ __forceinline__ void st_if(float *p, float v, bool on) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.f32 [%0], %1;\n\t}" ::"l"(p),
+               "f"(v), "r"((int)on)
+               : "memory");
+}
+__device__ __forceinline__ void red_add_if(float *p, float v, bool on) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p red.global.add.f32 [%0], %1;\n\t}" ::"l"(p),
+      "f"(v), "r"((int)on)
+      : "memory");
+}
+__device__ __forceinline__ float ldcg_if(const float *p, bool on) {
+  float v;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+      "@p ld.global.cg.f32 %0, [%1];\n\t}"
+      : "=f"(v)
+      : "l"(p), "r"((int)on)
+      : "memory");
+  return v;
+}
+
+// 16 bytes to a 16-byte aligned shared-memory address
+__device__ __forceinline__ void sts128(uint32_t saddr, const uint4 &v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(v.x), "r"(v.y),
+               "r"(v.z), "r"(v.w)
+               : "memory");
+}
+
 }  // namespace ls
