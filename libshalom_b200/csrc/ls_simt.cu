@@ -94,64 +94,6 @@ k_gemm_strided(GemmArgs<T> g, long sA, long sB, long sC, long count,
   }
 }
 
-template <typename T> struct EntryOf;
-template <> struct EntryOf<float> { using type = LibShalom_sgemm_entry; };
-template <> struct EntryOf<double> { using type = LibShalom_dgemm_entry; };
-
-// Grouped batch.  Work unit = a run of consecutive entries naming the same C
-// (a single entry is a run of one).  CTAs take entry indices from an atomic
-// counter; an index that continues a run is skipped (its run's owner
-// processes it), so every C block is owned by exactly one CTA and the
-// products of a run are applied in array order.
-template <typename T, class Cfg>
-__global__ void __launch_bounds__(Cfg::NTH)
-k_gemm_grouped(const typename EntryOf<T>::type *entries, long count,
-               unsigned long long *counter) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *smem = reinterpret_cast<T *>(smem_raw);
-  __shared__ long s_idx;
-  for (;;) {
-    if (threadIdx.x == 0) {
-      long i = (long)atomicAdd(counter, 1ULL);
-      // skip indices that continue a run
-      while (i < count && i > 0 && entries[i].C == entries[i - 1].C)
-        i = (long)atomicAdd(counter, 1ULL);
-      s_idx = i;
-    }
-    __syncthreads();
-    const long first = s_idx;
-    __syncthreads();
-    if (first >= count) break;
-    long last = first + 1;
-    while (last < count && entries[last].C == entries[first].C) ++last;
-
-    const auto &e0 = entries[first];
-    const int tiles_m = (e0.M + Cfg::BM - 1) / Cfg::BM;
-    const int tiles_n = (e0.N + Cfg::BN - 1) / Cfg::BN;
-    for (int t = 0; t < tiles_m * tiles_n; ++t) {
-      for (long p = first; p < last; ++p) {
-        const auto &e = entries[p];
-        GemmArgs<T> h;
-        h.A = e.A; h.B = e.B; h.C = e.C;
-        h.M = e.M; h.N = e.N; h.K = e.K;
-        h.transa = 0; h.transb = e.transb;
-        h.lda = e.lda > 0 ? e.lda : e.K;
-        h.ldb = e.ldb > 0 ? e.ldb : (e.transb ? e.K : e.N);
-        h.ldc = e.ldc > 0 ? e.ldc : e.N;
-        h.alpha = (T)e.alpha; h.beta = (T)e.beta;
-        if (h.transb)
-          simt_tile<T, Cfg, 0, false, true>(h, (long)(t / tiles_n) * Cfg::BM,
-                                            (long)(t % tiles_n) * Cfg::BN, 0, h.K, h.C, h.ldc,
-                                            h.alpha, h.beta, smem);
-        else
-          simt_tile<T, Cfg, 0, false, false>(h, (long)(t / tiles_n) * Cfg::BM,
-                                             (long)(t % tiles_n) * Cfg::BN, 0, h.K, h.C, h.ldc,
-                                             h.alpha, h.beta, smem);
-      }
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
 // tile configurations
 // ---------------------------------------------------------------------------
@@ -413,9 +355,10 @@ static int launch_strided(const GemmArgs<T> &g, long sA, long sB, long sC, long 
 
 template <>
 int run_strided<float>(const GemmArgs<float> &g, long sA, long sB, long sC, long count) {
-  if (g.M <= 32 && g.N <= 32) return launch_strided<float, S32>(g, sA, sB, sC, count, 6);
-  if (g.M <= 64 && g.N <= 64) return launch_strided<float, S64>(g, sA, sB, sC, count, 4);
-  return launch_strided<float, S128>(g, sA, sB, sC, count, 1);
+  // (64-bit sizes: beyond the int32 indices of the flexible tiles)
+  const long most = std::max({g.M, g.N, g.K, g.lda, g.ldb, g.ldc});
+  if (most >= (1L << 30)) return launch_strided<float, S64>(g, sA, sB, sC, count, 4);
+  return run_flex_strided(g, sA, sB, sC, count);
 }
 template <>
 int run_strided<double>(const GemmArgs<double> &g, long sA, long sB, long sC, long count) {
@@ -423,34 +366,10 @@ int run_strided<double>(const GemmArgs<double> &g, long sA, long sB, long sC, lo
   return launch_strided<double, D64>(g, sA, sB, sC, count, 2);
 }
 
-template <typename T, class Cfg>
-static int launch_grouped(const typename EntryOf<T>::type *entries, long count, int per_sm) {
-  void *ws = nullptr;
-  int rc = workspace(64, &ws);
-  if (rc) return rc;
-  unsigned long long *counter = reinterpret_cast<unsigned long long *>(ws);
-  LS_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), state().stream));
-  const size_t smem = smem_of<T, Cfg>();
-  auto kern = k_gemm_grouped<T, Cfg>;
-  per_sm = occupancy_of((const void *)kern, Cfg::NTH, smem, per_sm);
-  const int grid = grid_for(count, per_sm);
-  kern<<<grid, Cfg::NTH, smem, state().stream>>>(entries, count, counter);
-  LS_CUDA_TRY(cudaGetLastError());
-  return LIBSHALOM_SUCCESS;
-}
-
-int run_grouped_s(const LibShalom_sgemm_entry *entries, long count) {
-  return launch_grouped<float, S64>(entries, count, 4);
-}
 // Grouped FP64 batches go to the run kernel of ls_dgemm.cu (C tile held in
-// registers across a run, cp.async double buffer); the generic tile kernel
-// above stays available for comparison.
+// registers across a run, cp.async double buffer).
 int run_grouped_d(const LibShalom_dgemm_entry *entries, long count) {
   return run_dgemm_runs(entries, count);
-}
-
-int run_grouped_d_generic(const LibShalom_dgemm_entry *entries, long count) {
-  return launch_grouped<double, D32>(entries, count, 4);
 }
 
 }  // namespace ls

@@ -1,0 +1,281 @@
+// ls_simt_flex.cu -- uniform and grouped batches of plain FP32 products
+// (LibShalom_sgemm_batched_strided, LibShalom_sgemm_batched) on the tiles of
+// ls_flex.cuh: many CTAs of 128 threads per SM, each computing one tile at a
+// time.
+#include <algorithm>
+
+#include "ls_common.cuh"
+#include "ls_flex.cuh"
+#include "ls_simt_launch.h"
+
+namespace ls {
+
+namespace {
+
+using F64 = FlexCfg<64, 64>;
+using F128 = FlexCfg<64, 128>;
+
+// edge of tile t of `tiles` that cover `n` evenly, in steps of 4
+__host__ __device__ __forceinline__ int flex_edge(int n, int tiles) {
+  return ((n + tiles - 1) / tiles + 3) / 4 * 4;
+}
+
+// ---------------------------------------------------------------------------
+// uniform batches: work item = (product, tile)
+// ---------------------------------------------------------------------------
+struct FlexUniform {
+  const float *A, *B;
+  float *C;
+  long sA, sB, sC, items;
+  int M, N, K, lda, ldb, ldc, transb;
+  float alpha, beta;
+  int tiles, tiles_n, edge_m, edge_n;
+};
+
+template <class Cfg, int TM, int TN, int PER_SM>
+__global__ void __launch_bounds__(FX_THREADS, PER_SM) k_flex_uniform(const FlexUniform u) {
+  extern __shared__ __align__(16) float fsm[];
+  FlexJob j;
+  j.K = u.K;
+  j.lda = u.lda; j.ldb = u.ldb; j.ldc = u.ldc; j.transb = u.transb;
+  j.alpha = u.alpha; j.beta = u.beta;
+  for (long w = blockIdx.x; w < u.items; w += gridDim.x) {
+    const long g = u.tiles == 1 ? w : w / u.tiles;
+    const int t = (int)(w - g * u.tiles), tm = u.tiles_n == 1 ? t : t / u.tiles_n;
+    const int m0 = tm * u.edge_m, n0 = (t - tm * u.tiles_n) * u.edge_n;
+    j.A = u.A + g * u.sA; j.B = u.B + g * u.sB; j.C = u.C + g * u.sC;
+    flex_tile<Cfg, TM, TN>(j, m0, n0, min(u.edge_m, u.M - m0), min(u.edge_n, u.N - n0), fsm);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// grouped batches
+// ---------------------------------------------------------------------------
+constexpr int FG_CLASSES = 64;  // work classes: half octaves of M N K a part
+constexpr int FG_PARTS = 16;    // a run's tiles are dealt to at most 16 items
+constexpr unsigned FG_LONG = (1u << 28) - 1;  // products of a run an item word can hold
+
+// Plan: every run of entries sharing C becomes min(tiles, parts) items {first
+// entry, products << 4 | part}, counting-sorted heaviest first, in two lists:
+// C of more than 64 columns and 32 rows takes 64 x 128 tiles of 8 x 8 outputs
+// a thread, the rest 64 x 64 tiles of 8 x 4 or 4 x 4 (one list for all: 1.57 ms
+// on 50,000 products of 4..256, two lists 1.51 ms; one CTA a run on 64 x 64
+// tiles, as before: 4.66 ms).  The lists fill one array from its two ends.
+struct FlexPlan {
+  unsigned *class_n, *class_off, *class_fill;  // [2][FG_CLASSES]: small, wide
+  unsigned *n_items, *counter;                 // [2]
+  uint2 *items;  // [n]: small ones upwards from 0, wide ones downwards from n - 1
+  long n;        // parts * count
+  int parts;
+};
+
+__device__ __forceinline__ bool fg_wide(int M, int N) { return M > 32 && N > 64; }
+__device__ __forceinline__ void fg_tiles(int M, int N, int *tiles_m, int *tiles_n) {
+  *tiles_m = (M + 63) / 64;
+  *tiles_n = fg_wide(M, N) ? (N + 127) / 128 : (N + 63) / 64;
+}
+
+// items, class and length of the run starting at entry i (0 items: empty C)
+__device__ __forceinline__ int fg_run(const LibShalom_sgemm_entry *e, long count, long i,
+                                      int max_parts, long *len, int *cls) {
+  const int M = e[i].M, N = e[i].N;
+  long k = 0, j = i;
+  do {
+    k += 16 + max(0, e[j].K);  // each product costs about 16 k of overhead
+    ++j;
+  } while (j < count && e[j].C == e[i].C);
+  *len = j - i;
+  *cls = 0;
+  if (M <= 0 || N <= 0) return 0;
+  int tm, tn;
+  fg_tiles(M, N, &tm, &tn);
+  const int parts = (int)min((long)tm * tn, (long)max_parts);
+  const float work = (float)M * (float)N * (float)k / (float)parts;
+  *cls = max(0, min(FG_CLASSES - 1, (int)(2.0f * log2f(fmaxf(work, 1.0f)))));
+  if (fg_wide(M, N)) *cls += FG_CLASSES;
+  return parts;
+}
+
+__global__ void k_fg_count(const LibShalom_sgemm_entry *e, long count, FlexPlan pl) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count;
+       i += (long)gridDim.x * blockDim.x) {
+    if (i > 0 && e[i].C == e[i - 1].C) continue;
+    long len;
+    int cls;
+    const int parts = fg_run(e, count, i, pl.parts, &len, &cls);
+    if (parts) atomicAdd(&pl.class_n[cls], (unsigned)parts);
+  }
+}
+
+__global__ void __launch_bounds__(2 * FG_CLASSES) k_fg_offsets(FlexPlan pl) {
+  __shared__ unsigned n[2 * FG_CLASSES];
+  const int c = threadIdx.x, list = c / FG_CLASSES, lo = list * FG_CLASSES;
+  n[c] = pl.class_n[c];
+  __syncthreads();
+  unsigned before = 0;
+  for (int i = lo + FG_CLASSES - 1; i > c; --i) before += n[i];
+  pl.class_off[c] = before;
+  if (c == lo) pl.n_items[list] = before + n[c];
+}
+
+__global__ void k_fg_place(const LibShalom_sgemm_entry *e, long count, FlexPlan pl) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count;
+       i += (long)gridDim.x * blockDim.x) {
+    if (i > 0 && e[i].C == e[i - 1].C) continue;
+    long len;
+    int cls;
+    const int parts = fg_run(e, count, i, pl.parts, &len, &cls);
+    if (!parts) continue;
+    const unsigned slot = pl.class_off[cls] + atomicAdd(&pl.class_fill[cls], (unsigned)parts);
+    const unsigned n = (unsigned)min(len, (long)FG_LONG);
+    for (int p = 0; p < parts; ++p) {
+      const long at = (long)slot + p;
+      pl.items[cls < FG_CLASSES ? at : pl.n - 1 - at] = make_uint2((unsigned)i, n << 4 | (unsigned)p);
+    }
+  }
+}
+
+// CTAs take items from a counter.  Thread 0 keeps two items ahead: the list
+// word of the next item and the counter value after it are in flight while an
+// item is computed (inline PTX: the compiler would aggregate an atomicAdd over
+// the warp and wait for its result on the spot).
+template <bool WIDE>
+__global__ void __launch_bounds__(FX_THREADS, WIDE ? 4 : 6)
+    k_flex_grouped(const LibShalom_sgemm_entry *entries, long count, FlexPlan pl) {
+  extern __shared__ __align__(16) float fsm[];
+  __shared__ uint2 s_item[2];
+  const unsigned n_items = pl.n_items[WIDE];
+  uint2 nxt = make_uint2(0, 0);
+  unsigned idx = 0;
+  auto take = [&]() {
+    asm volatile("atom.global.add.u32 %0, [%1], 1;"
+                 : "=r"(idx)
+                 : "l"(pl.counter + WIDE)
+                 : "memory");
+  };
+  auto at = [&](long i) { return pl.items[WIDE ? pl.n - 1 - i : i]; };
+  if (threadIdx.x == 0) {
+    s_item[0] = blockIdx.x < n_items ? at(blockIdx.x) : make_uint2(0, 0);
+    const unsigned i1 = blockIdx.x + gridDim.x;
+    if (i1 < n_items) nxt = at(i1);
+    take();
+  }
+  __syncthreads();
+  for (int it = 0;; it ^= 1) {
+    const uint2 item = s_item[it];
+    if (item.y == 0) break;  // no products: past the list
+    if (threadIdx.x == 0) {
+      s_item[it ^ 1] = nxt;
+      nxt = make_uint2(0, 0);
+      const unsigned long i2 = 2ul * gridDim.x + idx;
+      if (i2 < n_items) {
+        nxt = at((long)i2);
+        take();
+      }
+    }
+    const LibShalom_sgemm_entry *run = entries + item.x;
+    const long most = count - item.x;  // (a run as long as FG_LONG: up to its end)
+    const unsigned len = item.y >> 4;
+    const int M = run->M, N = run->N;
+    int tiles_m, tiles_n;
+    fg_tiles(M, N, &tiles_m, &tiles_n);
+    const int em = flex_edge(M, tiles_m), en = flex_edge(N, tiles_n);
+    for (long t = item.y & (FG_PARTS - 1); t < (long)tiles_m * tiles_n; t += pl.parts) {
+      const int tm = (int)(t / tiles_n), tn = (int)(t - (long)tm * tiles_n);
+      const int m0 = tm * em, n0 = tn * en, mrows = min(em, M - m0), ncols = min(en, N - n0);
+      if (mrows <= 0 || ncols <= 0) continue;
+      const bool small = ((mrows + 3) >> 2) * ((ncols + 3) >> 2) <= FX_THREADS;
+      for (long p = 0; p < len || (len == FG_LONG && p < most && run[p].C == run->C); ++p) {
+        const LibShalom_sgemm_entry &e = run[p];
+        FlexJob j;
+        j.A = e.A; j.B = e.B; j.C = e.C;
+        j.K = max(0, e.K); j.transb = e.transb;
+        j.lda = e.lda > 0 ? e.lda : j.K;
+        j.ldb = e.ldb > 0 ? e.ldb : (e.transb ? j.K : N);
+        j.ldc = e.ldc > 0 ? e.ldc : N;
+        j.alpha = e.alpha; j.beta = e.beta;
+        if constexpr (WIDE) flex_tile<F128, 8, 8>(j, m0, n0, mrows, ncols, fsm);
+        else if (small) flex_tile<F64, 4, 4>(j, m0, n0, mrows, ncols, fsm);
+        else flex_tile<F64, 8, 4>(j, m0, n0, mrows, ncols, fsm);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <class Cfg, int TM, int TN, int PER_SM>
+int launch_uniform(FlexUniform &u, long count) {
+  const int tiles_m = (int)cdiv(u.M, Cfg::MAXM);
+  u.tiles_n = (int)cdiv(u.N, Cfg::MAXN);
+  u.edge_m = flex_edge(u.M, tiles_m);
+  u.edge_n = flex_edge(u.N, u.tiles_n);
+  // edges in steps of 4 can leave the last tile empty
+  u.tiles_n = (int)cdiv(u.N, u.edge_n);
+  u.tiles = (int)cdiv(u.M, u.edge_m) * u.tiles_n;
+  u.items = (long)u.tiles * count;
+  auto kern = k_flex_uniform<Cfg, TM, TN, PER_SM>;
+  const int per_sm = occupancy_of((const void *)kern, FX_THREADS, Cfg::SMEM, PER_SM);
+  kern<<<grid_for(u.items, per_sm), FX_THREADS, Cfg::SMEM, state().stream>>>(u);
+  LS_CUDA_TRY(cudaGetLastError());
+  return LIBSHALOM_SUCCESS;
+}
+
+}  // namespace
+
+int run_flex_strided(const GemmArgs<float> &g, long sA, long sB, long sC, long count) {
+  FlexUniform u{};
+  u.A = g.A; u.B = g.B; u.C = g.C;
+  u.sA = sA; u.sB = sB; u.sC = sC;
+  u.M = (int)g.M; u.N = (int)g.N; u.K = (int)g.K;
+  u.lda = (int)g.lda; u.ldb = (int)g.ldb; u.ldc = (int)g.ldc;
+  u.transb = g.transb;
+  u.alpha = g.alpha; u.beta = g.beta;
+  // the smallest thread tile that covers a product in one CTA, 8 x 8 (fewest
+  // shared-memory loads per FMA) beyond 64 columns.  B200, 10,000 products
+  // against the fixed 32 / 64 / 128 tiles before: 24^3 NN 49 (74) us, 33^3 NN 90
+  // (217), 64^3 NN 198 (213), 72^3 NT 495 (959), 104^3 NT 959 (1,241)
+  if (cdiv(g.M, 4) * cdiv(g.N, 4) <= FX_THREADS && g.M <= 64 && g.N <= 64)
+    return launch_uniform<F64, 4, 4, 6>(u, count);
+  if (g.N <= 64) return launch_uniform<F64, 8, 4, 6>(u, count);
+  return launch_uniform<F128, 8, 8, 4>(u, count);
+}
+
+int run_grouped_s(const LibShalom_sgemm_entry *entries, long count) {
+  State &st = state();
+  if (count > UINT32_MAX) return LIBSHALOM_ERR_UNSUPPORTED;
+  const size_t header = 512;
+  FlexPlan pl;
+  // one item a run where the items would take much memory
+  pl.parts = count <= (1L << 22) ? FG_PARTS : 1;
+  void *ws = nullptr;
+  int rc = workspace((header + 2 * (size_t)pl.parts * (size_t)count) * sizeof(unsigned), &ws);
+  if (rc && pl.parts > 1) {
+    pl.parts = 1;
+    rc = workspace((header + 2 * (size_t)count) * sizeof(unsigned), &ws);
+  }
+  if (rc) return rc;
+  unsigned *w = static_cast<unsigned *>(ws);
+  pl.n = pl.parts * count;
+  pl.class_n = w;
+  pl.class_off = w + 2 * FG_CLASSES;
+  pl.class_fill = w + 4 * FG_CLASSES;
+  pl.n_items = w + 6 * FG_CLASSES;
+  pl.counter = pl.n_items + 2;
+  pl.items = reinterpret_cast<uint2 *>(w + header);
+  LS_CUDA_TRY(cudaMemsetAsync(w, 0, header * sizeof(unsigned), st.stream));
+  const int pgrid = (int)std::max(1L, std::min(cdiv(count, 256), (long)st.num_sms * 8));
+  k_fg_count<<<pgrid, 256, 0, st.stream>>>(entries, count, pl);
+  k_fg_offsets<<<1, 2 * FG_CLASSES, 0, st.stream>>>(pl);
+  k_fg_place<<<pgrid, 256, 0, st.stream>>>(entries, count, pl);
+  LS_CUDA_TRY(cudaGetLastError());
+  const int ps_w = occupancy_of((const void *)k_flex_grouped<true>, FX_THREADS, F128::SMEM, 4);
+  const int ps_s = occupancy_of((const void *)k_flex_grouped<false>, FX_THREADS, F64::SMEM, 6);
+  k_flex_grouped<true><<<grid_for((long)st.num_sms * ps_w, ps_w), FX_THREADS, F128::SMEM,
+                         st.stream>>>(entries, count, pl);
+  k_flex_grouped<false><<<grid_for((long)st.num_sms * ps_s, ps_s), FX_THREADS, F64::SMEM,
+                          st.stream>>>(entries, count, pl);
+  LS_CUDA_TRY(cudaGetLastError());
+  return LIBSHALOM_SUCCESS;
+}
+
+}  // namespace ls
