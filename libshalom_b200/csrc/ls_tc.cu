@@ -564,11 +564,15 @@ constexpr int W_CONV0 = 2, N_CONV = 8;
 // Warp roles of k_tc_ws: warp 0 producer, warp 1 MMA, then NC converter and
 // NE epilogue warps.  WIDE (short K, C written by TMA stores): 16 converters
 // and 4 epilogue warps (one per TMEM lane quarter), since the split is the
-// busiest role there.  Otherwise 8 + 8: long-K tiles hold the register fold of
+// busiest role there.  NARROW (long K on tiles of at most 64 columns): two
+// groups of 8 converters that take alternate slabs, one BF16 buffer each; one
+// group of 8 spent 890 of a slab's 1,210 cycles on its chain of load, split,
+// store and hand-off.  Otherwise 8 + 8: long-K tiles hold the register fold of
 // 64 columns per epilogue thread, and packed small GEMMs store C row by row.
-template <bool WIDE>
+template <bool WIDE, bool NARROW>
 struct WsRoles {
-  static constexpr int NC = WIDE ? 16 : 8;
+  static constexpr int NC = WIDE || NARROW ? 16 : 8;
+  static constexpr int CG = NARROW ? 2 : 1;  // converter groups
   static constexpr int NE = WIDE ? 4 : 8;
   static constexpr int W_EPI = 2 + NC;
   static constexpr int THREADS = (2 + NC + NE) * 32;
@@ -577,8 +581,57 @@ struct WsRoles {
 constexpr int WS_TMEM_COLS = 512;  // 2 x (D_main 128 + D_corr 128)
 
 // mbarrier slots (8 bytes each) after WS_OFF_BAR
-enum { B_FULL = 0, B_EMPTY = 4, B_BFULL = 8, B_BEMPTY = 10, B_AFULL = 12, B_AEMPTY = 14,
-       B_FINAL = 16, B_COUNT = 17 };
+enum { B_FULL = 0, B_EMPTY = 8, B_BFULL = 16, B_BEMPTY = 18, B_AFULL = 20, B_AEMPTY = 22,
+       B_FINAL = 24, B_COUNT = 25 };
+static_assert(8 * B_COUNT + 8 <= 256, "barriers, TMEM address and abort flag");
+
+// Shared-memory layout.  NARROW (long K on tiles of at most 64 columns): the
+// FP32 stages shrink with the tile and A's BF16 parts are in TMEM, so there is
+// room for 8 stages.
+//
+// A narrow tile multiplies little and moves much: per slab of 32 k the
+// shared-memory pipe carried 60 KB of MMA operand reads, 50 KB of converter
+// traffic and 20 KB of TMA writes for 128 x 32 outputs.  20480 x 32 x 20480 on
+// a B200, step by step: 568 us; more stages 560; A's parts in TMEM (the MMAs
+// read no A from shared memory, the converters write none) 488; two converter
+// groups 455; op(B)'s parts side by side (6 MMAs a slab instead of 12) 433 (452 sustained).
+// Bound now by the MMA warp's chain of wait, issue and commit (about 1,000
+// cycles a slab) on schedulers it shares with the converters.
+template <bool NARROW>
+struct WsLayout {
+  // BF16 buffers: [split][A | B][chunk][row]; NARROW: op(B) alone, as
+  // [chunk][split][row]
+  static constexpr int SPLIT = SPLIT_BYTES;
+  static constexpr int BUF = NARROW ? 4 * 3 * 64 * 16 : BUF_BYTES;
+  static constexpr int OFF_STAGE = 2 * BUF;
+  static constexpr int ROOM = WS_OFF_CST - OFF_STAGE;
+  // bytes of a stage and their number, for tiles of tn columns
+  static __host__ __device__ constexpr int stage_bytes(int tn) {
+    return NARROW ? 16384 + tn * 128 : WS_STAGE_BYTES;
+  }
+  static __host__ __device__ constexpr int stages(int tn) {
+    return ROOM / stage_bytes(tn) < 8 ? ROOM / stage_bytes(tn) : 8;
+  }
+  static_assert(OFF_STAGE % 1024 == 0, "swizzled boxes");
+};
+static_assert(WsLayout<false>::OFF_STAGE == WS_OFF_STAGE && WsLayout<false>::stages(128) == WS_STAGES);
+
+// NARROW: A's BF16 parts live in TMEM, beside the accumulators (three blocks
+// of at most 64 columns a set): buffer b at TM_A + b * 256, 16 columns a part
+// (8 a k-step)
+constexpr uint32_t TM_A = 192;
+
+// Running position in a ring of n stages
+struct RingPos {
+  int st = 0;
+  uint32_t phase = 0;  // of the ring's current round
+  __device__ __forceinline__ void next(int n) {
+    if (++st == n) {
+      st = 0;
+      phase ^= 1;
+    }
+  }
+};
 
 struct WsArgs {
   TcProblem p;
@@ -596,11 +649,86 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
       : "memory");
 }
 
+// The MMAs of one slab from BF16 buffer B into accumulator set ACC (one lane).
+// TMEM starts at 0: the kernels that use this allocate all 512 columns.
+// SWAP: op(B) is the 128-row operand.
+template <int NSPLIT, bool SWAP, class L, int B, int ACC>
+__device__ __forceinline__ void tc_issue_slab(uint32_t smem_base, uint32_t idesc, uint32_t first,
+                                              bool two) {
+  const uint32_t bb = smem_base + WS_OFF_BUF + B * L::BUF;
+  constexpr uint32_t dm = ACC * 256, dc = dm + 128;
+#pragma unroll
+  for (int ks = 0; ks < 2; ++ks) {
+    if (ks == 1 && !two) break;
+    uint64_t a[3], b[3];
+#pragma unroll
+    for (int sp = 0; sp < NSPLIT; ++sp) {
+      a[sp] = ptx::smem_desc(bb + sp * L::SPLIT + ks * 2 * CHUNK_BYTES, CHUNK_BYTES, 128);
+      b[sp] = ptx::smem_desc(bb + sp * L::SPLIT + 8192 + ks * 2 * CHUNK_BYTES, CHUNK_BYTES, 128);
+    }
+    const uint32_t acc = ks == 0 ? first : 1u;
+    auto mma = [&](uint32_t d, int i, int k, uint32_t accumulate) {
+      ptx::mma_bf16(d, SWAP ? b[i] : a[i], SWAP ? a[k] : b[k], idesc, accumulate);
+    };
+    mma(dm, 0, 0, acc);
+    mma(dc, 0, 1, acc);
+    mma(dc, 1, 0, 1u);
+    if (NSPLIT == 3) {
+      mma(dc, 0, 2, 1u);
+      mma(dc, 2, 0, 1u);
+      mma(dc, 1, 1, 1u);
+    }
+  }
+}
+// The same for a NARROW tile of tn columns: A's parts in TMEM, op(B)'s parts
+// one after the other along the MMA's N, so that part i of A multiplies all
+// the parts of op(B) it needs in one MMA.  The set holds D_main (hi hi) and two
+// correction blocks of tn columns, (hi mid + mid hi) and (hi lo + mid mid + lo
+// hi).
+template <int NSPLIT, int B, int ACC>
+__device__ __forceinline__ void tc_issue_narrow(uint32_t smem_base, int tn, uint32_t first,
+                                                bool two) {
+  const uint32_t bb = smem_base + WS_OFF_BUF + B * WsLayout<true>::BUF;
+  const uint32_t chunk = NSPLIT * 16 * tn;
+#pragma unroll
+  for (int ks = 0; ks < 2; ++ks) {
+    if (ks == 1 && !two) break;
+    const uint64_t b = ptx::smem_desc(bb + ks * 2 * chunk, chunk, 128);
+#pragma unroll
+    for (int sp = 0; sp < NSPLIT; ++sp)
+      ptx::mma_bf16_ts(ACC * 256 + sp * tn, TM_A + B * 256 + sp * 16 + ks * 8, b,
+                       ptx::idesc_bf16_f32(TC_BM, (NSPLIT - sp) * tn),
+                       ks == 0 && sp == 0 ? first : 1u);
+  }
+}
+template <int NSPLIT>
+__device__ __forceinline__ void tc_issue_narrow(int buf, int acc, uint32_t smem_base, int tn,
+                                                uint32_t first, bool two) {
+  if (buf == 0) {
+    if (acc == 0) tc_issue_narrow<NSPLIT, 0, 0>(smem_base, tn, first, two);
+    else tc_issue_narrow<NSPLIT, 0, 1>(smem_base, tn, first, two);
+  } else {
+    if (acc == 0) tc_issue_narrow<NSPLIT, 1, 0>(smem_base, tn, first, two);
+    else tc_issue_narrow<NSPLIT, 1, 1>(smem_base, tn, first, two);
+  }
+}
+template <int NSPLIT, bool SWAP, class L>
+__device__ __forceinline__ void tc_issue(int buf, int acc, uint32_t smem_base, uint32_t idesc,
+                                         uint32_t first, bool two) {
+  if (buf == 0) {
+    if (acc == 0) tc_issue_slab<NSPLIT, SWAP, L, 0, 0>(smem_base, idesc, first, two);
+    else tc_issue_slab<NSPLIT, SWAP, L, 0, 1>(smem_base, idesc, first, two);
+  } else {
+    if (acc == 0) tc_issue_slab<NSPLIT, SWAP, L, 1, 0>(smem_base, idesc, first, two);
+    else tc_issue_slab<NSPLIT, SWAP, L, 1, 1>(smem_base, idesc, first, two);
+  }
+}
+
 // BLX > 0: each epilogue warp holds at most BLX 32-column blocks of C (a
 // DRAIN kernel for tiles of at most 32 * BLX * (epilogue warps / 4) columns
 // keeps a smaller register fold)
 template <int NSPLIT, bool DRAIN, bool WIDE, int BLX = 0>
-__global__ void __launch_bounds__(WsRoles<WIDE>::THREADS, 1)
+__global__ void __launch_bounds__(WsRoles<WIDE, (BLX == 1)>::THREADS, 1)
     k_tc_ws(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ CUtensorMap tmC, const WsArgs args) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -613,15 +741,17 @@ __global__ void __launch_bounds__(WsRoles<WIDE>::THREADS, 1)
   const int tn = p.tile_n;
   const int kc = DRAIN ? p.kc_slabs : (1 << 30);
   static_assert(!(DRAIN && WIDE), "the long-K fold needs 8 epilogue warps");
-  using Roles = WsRoles<WIDE>;
+  using Roles = WsRoles<WIDE, (BLX == 1)>;
+  using L = WsLayout<(BLX == 1)>;
+  const int nst = L::stages(tn), stage_bytes = L::stage_bytes(tn);
 
   if (tid == 0) {
-    for (int i = 0; i < WS_STAGES; ++i) {
+    for (int i = 0; i < nst; ++i) {
       ptx::mbar_init(&bars[B_FULL + i], 1);
-      ptx::mbar_init(&bars[B_EMPTY + i], Roles::NC);
+      ptx::mbar_init(&bars[B_EMPTY + i], Roles::NC / Roles::CG);
     }
     for (int i = 0; i < 2; ++i) {
-      ptx::mbar_init(&bars[B_BFULL + i], Roles::NC);
+      ptx::mbar_init(&bars[B_BFULL + i], Roles::NC / Roles::CG);
       ptx::mbar_init(&bars[B_BEMPTY + i], 1);
       ptx::mbar_init(&bars[B_AFULL + i], 1);
       ptx::mbar_init(&bars[B_AEMPTY + i], Roles::NE);
@@ -643,14 +773,13 @@ __global__ void __launch_bounds__(WsRoles<WIDE>::THREADS, 1)
     // ------------------------------ producer ------------------------------
     if (lane == 0) {
       long j = 0;
+      RingPos r;
       for (long t = blockIdx.x; t < p.num_tiles && !*s_abort; t += gridDim.x) {
         const TileInfo ti = decode_tile(p, t);
-        for (int s = 0; s < p.nk; ++s, ++j) {
-          const int st = (int)(j % WS_STAGES);
-          if (j >= WS_STAGES &&
-              !ws_wait(&bars[B_EMPTY + st], (uint32_t)(((j / WS_STAGES) - 1) & 1), s_abort, p.err))
-            break;
-          const uint32_t dst = smem_base + WS_OFF_STAGE + st * WS_STAGE_BYTES;
+        for (int s = 0; s < p.nk; ++s, ++j, r.next(nst)) {
+          const int st = r.st;
+          if (j >= nst && !ws_wait(&bars[B_EMPTY + st], r.phase ^ 1, s_abort, p.err)) break;
+          const uint32_t dst = smem_base + L::OFF_STAGE + st * stage_bytes;
           mbar_arrive_tx(&bars[B_FULL + st], args.tx_bytes);
           const int k0 = s * TC_BK;
           // split-K: slice g reads K range [g*kslice, (g+1)*kslice) of one matrix
@@ -670,8 +799,8 @@ __global__ void __launch_bounds__(WsRoles<WIDE>::THREADS, 1)
     long j = 0, u = 0;
     bool ok = true;
     for (long t = blockIdx.x; ok && t < p.num_tiles; t += gridDim.x) {
+      int s_in = 0;  // slab of the accumulation chunk
       for (int s = 0; s < p.nk; ++s, ++j) {
-        const int s_in = s % kc;
         // new accumulation chunk: wait until the epilogue has drained this set
         if (s_in == 0 && u >= 2)
           ok = ws_wait(&bars[B_AEMPTY + (u & 1)], (uint32_t)(((u >> 1) - 1) & 1), s_abort, p.err);
@@ -682,34 +811,18 @@ __global__ void __launch_bounds__(WsRoles<WIDE>::THREADS, 1)
         ptx::tc_fence_after();
         const bool last = s_in == kc - 1 || s == p.nk - 1;
         if (ptx::elect_one()) {
-          const uint32_t acc_base = tmem + (uint32_t)((u & 1) * 256);
-          const uint32_t bb = smem_base + WS_OFF_BUF + b * BUF_BYTES;
-          const int ksteps = min(2, (p.K - s * TC_BK + 15) / 16);
-#pragma unroll
-          for (int ks = 0; ks < 2; ++ks) {
-            if (ks >= ksteps) break;
-            const uint32_t acc = (s_in > 0 || ks > 0) ? 1u : 0u;
-            uint64_t da[3], db[3];
-#pragma unroll
-            for (int sp = 0; sp < NSPLIT; ++sp) {
-              da[sp] = ptx::smem_desc(bb + sp * SPLIT_BYTES + ks * 2 * CHUNK_BYTES, CHUNK_BYTES, 128);
-              db[sp] = ptx::smem_desc(bb + sp * SPLIT_BYTES + 8192 + ks * 2 * CHUNK_BYTES,
-                                      CHUNK_BYTES, 128);
-            }
-            ptx::mma_bf16(acc_base, da[0], db[0], idesc, acc);
-            ptx::mma_bf16(acc_base + 128, da[0], db[1], idesc, acc);
-            ptx::mma_bf16(acc_base + 128, da[1], db[0], idesc, 1u);
-            if (NSPLIT == 3) {
-              ptx::mma_bf16(acc_base + 128, da[0], db[2], idesc, 1u);
-              ptx::mma_bf16(acc_base + 128, da[2], db[0], idesc, 1u);
-              ptx::mma_bf16(acc_base + 128, da[1], db[1], idesc, 1u);
-            }
-          }
+          const uint32_t acc = s_in > 0 ? 1u : 0u;
+          const bool two = p.K - s * TC_BK > 16;
+          if constexpr (BLX == 1)
+            tc_issue_narrow<NSPLIT>(b, (int)(u & 1), smem_base, tn, acc, two);
+          else
+            tc_issue<NSPLIT, false, L>(b, (int)(u & 1), smem_base, idesc, acc, two);
           ptx::mma_commit(&bars[B_BEMPTY + b]);  // operand buffer b may be refilled
           if (last) ptx::mma_commit(&bars[B_AFULL + (u & 1)]);  // accumulation chunk complete
         }
         __syncwarp();
         if (last) ++u;
+        s_in = last ? 0 : s_in + 1;
       }
     }
     // every MMA issued has completed before TMEM is freed
@@ -724,9 +837,9 @@ __global__ void __launch_bounds__(WsRoles<WIDE>::THREADS, 1)
     // tile's GEMMs and the chunks past K of a last half slab are not
     // converted: the MMA reads stale shared memory there, which reaches only
     // output rows and columns that are never stored (and no MMA k-step at all).
-    constexpr int NCT = Roles::NC * 32;
+    constexpr int NCT = Roles::NC / Roles::CG * 32;
     constexpr int PER = 512 / NCT;
-    const int ct = tid - W_CONV0 * 32;
+    const int ct = (tid - W_CONV0 * 32) % NCT, group = (tid - W_CONV0 * 32) / NCT;
     const bool nn = !p.transb;
     const int nn_w = args.nn_w;
     // quotients by tn and N through float reciprocals: exact for the ranges
@@ -734,42 +847,68 @@ __global__ void __launch_bounds__(WsRoles<WIDE>::THREADS, 1)
     // away from the next integer
     const float inv_tn = 1.0f / (float)tn, inv_n = 1.0f / (float)max(1, p.N);
     long j = 0;
+    RingPos r;
     bool ok = true;
     for (long t = blockIdx.x; ok && t < p.num_tiles; t += gridDim.x) {
       const TileInfo ti = decode_tile(p, t);
       const int a_rows = p.G > 1 ? ti.ng * p.M : min(TC_BM, p.M - ti.m0);
       const int b_cols = p.G > 1 ? ti.ng * p.N : min(tn, p.N - ti.n0);
-      for (int s = 0; s < p.nk; ++s, ++j) {
-        const int st = (int)(j % WS_STAGES), b = (int)(j & 1);
-        if (!ws_wait(&bars[B_FULL + st], (uint32_t)((j / WS_STAGES) & 1), s_abort, p.err)) {
-          ok = false;
-          break;
-        }
-        if (j >= 2 && !ws_wait(&bars[B_BEMPTY + b], (uint32_t)(((j >> 1) - 1) & 1), s_abort,
-                               p.err)) {
-          ok = false;
-          break;
-        }
+      for (int s = 0; s < p.nk; ++s, ++j, r.next(nst)) {
+        const int st = r.st, b = (int)(j & 1);
+        if (Roles::CG == 2 && b != group) continue;
+        // (warp-uniform: the TMEM stores below take the whole warp)
+        ok = ws_wait(&bars[B_FULL + st], r.phase, s_abort, p.err);
+        if (ok && j >= 2)
+          ok = ws_wait(&bars[B_BEMPTY + b], (uint32_t)(((j >> 1) - 1) & 1), s_abort, p.err);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
         const int nchunk = p.K - s * TC_BK <= 16 ? 2 : 4;  // the MMA's k-steps x 2
-        const unsigned char *stg = smem + WS_OFF_STAGE + st * WS_STAGE_BYTES;
-        unsigned char *base = smem + WS_OFF_BUF + b * BUF_BYTES;
+        const unsigned char *stg = smem + L::OFF_STAGE + st * stage_bytes;
+        unsigned char *base = smem + WS_OFF_BUF + b * L::BUF;
+        if constexpr (BLX == 1) {
+          // A's parts go to TMEM: the MMA reads A three times a k-step from
+          // there instead of six times from shared memory.  A warp reaches the
+          // 32 lanes of its number mod 4; every lane takes part (rows past the
+          // last hold the zeros of the TMA box)
+          if (j >= 2) ptx::tc_fence_after();
+          const int cr = (warp & 3) * 32 + lane, c0 = (ct >> 7) * 2;
+          const unsigned char *row = stg + cr * 128;
+          const uint32_t at = ((uint32_t)(warp & 3) << 21) + TM_A + b * 256;
 #pragma unroll
-        for (int q = 0; q < PER; ++q) {
-          const int idx = ct + q * NCT;
-          const int cr = idx & 127, c = idx >> 7;
-          if (cr < a_rows && c < nchunk) {
-            const unsigned char *row = stg + cr * 128;
-            const float4 u0 =
-                *reinterpret_cast<const float4 *>(row + (((2 * c) ^ (cr & 7)) << 4));
-            const float4 u1 =
-                *reinterpret_cast<const float4 *>(row + (((2 * c + 1) ^ (cr & 7)) << 4));
-            float x[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
-            uint4 h, m, l;
-            split8<NSPLIT>(x, h, m, l);
-            const int off = c * CHUNK_BYTES + cr * 16;
-            *reinterpret_cast<uint4 *>(base + off) = h;
-            *reinterpret_cast<uint4 *>(base + SPLIT_BYTES + off) = m;
-            if (NSPLIT == 3) *reinterpret_cast<uint4 *>(base + 2 * SPLIT_BYTES + off) = l;
+          for (int q = 0; q < 2; ++q) {
+            const int c = c0 + q;
+            if (c < nchunk) {
+              const float4 u0 =
+                  *reinterpret_cast<const float4 *>(row + (((2 * c) ^ (cr & 7)) << 4));
+              const float4 u1 =
+                  *reinterpret_cast<const float4 *>(row + (((2 * c + 1) ^ (cr & 7)) << 4));
+              float x[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+              uint4 h, m, l;
+              split8<NSPLIT>(x, h, m, l);
+              ptx::tmem_st4(at + c * 4, h);
+              ptx::tmem_st4(at + 16 + c * 4, m);
+              if (NSPLIT == 3) ptx::tmem_st4(at + 32 + c * 4, l);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < PER; ++q) {
+            const int idx = ct + q * NCT;
+            const int cr = idx & 127, c = idx >> 7;
+            if (cr < a_rows && c < nchunk) {
+              const unsigned char *row = stg + cr * 128;
+              const float4 u0 =
+                  *reinterpret_cast<const float4 *>(row + (((2 * c) ^ (cr & 7)) << 4));
+              const float4 u1 =
+                  *reinterpret_cast<const float4 *>(row + (((2 * c + 1) ^ (cr & 7)) << 4));
+              float x[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+              uint4 h, m, l;
+              split8<NSPLIT>(x, h, m, l);
+              const int off = c * CHUNK_BYTES + cr * 16;
+              *reinterpret_cast<uint4 *>(base + off) = h;
+              *reinterpret_cast<uint4 *>(base + L::SPLIT + off) = m;
+              if (NSPLIT == 3) *reinterpret_cast<uint4 *>(base + 2 * L::SPLIT + off) = l;
+            }
           }
         }
 #pragma unroll
@@ -800,11 +939,16 @@ __global__ void __launch_bounds__(WsRoles<WIDE>::THREADS, 1)
             }
             uint4 h, m, l;
             split8<NSPLIT>(x, h, m, l);
-            const int off = 8192 + c * CHUNK_BYTES + jj * 16;
+            const int off = BLX == 1 ? (c * NSPLIT * tn + jj) * 16 : 8192 + c * CHUNK_BYTES + jj * 16;
+            const int part = BLX == 1 ? tn * 16 : L::SPLIT;
             *reinterpret_cast<uint4 *>(base + off) = h;
-            *reinterpret_cast<uint4 *>(base + SPLIT_BYTES + off) = m;
-            if (NSPLIT == 3) *reinterpret_cast<uint4 *>(base + 2 * SPLIT_BYTES + off) = l;
+            *reinterpret_cast<uint4 *>(base + part + off) = m;
+            if (NSPLIT == 3) *reinterpret_cast<uint4 *>(base + 2 * part + off) = l;
           }
+        }
+        if constexpr (BLX == 1) {
+          ptx::tmem_wait_st();
+          ptx::tc_fence_before();
         }
         ptx::fence_proxy_async_smem();
         __syncwarp();
@@ -941,8 +1085,19 @@ __global__ void __launch_bounds__(WsRoles<WIDE>::THREADS, 1)
             if (ch >= c_lo && ch < c_hi) {
               float dm[8], dc[8];
               ptx::tmem_ld8(acc_base + ch * 8, dm);
-              ptx::tmem_ld8(acc_base + 128 + ch * 8, dc);
-              ptx::tmem_wait_ld();
+              if constexpr (BLX == 1) {
+                float d2[8];
+                ptx::tmem_ld8(acc_base + tn + ch * 8, dc);
+                if (NSPLIT == 3) ptx::tmem_ld8(acc_base + 2 * tn + ch * 8, d2);
+                ptx::tmem_wait_ld();
+                if (NSPLIT == 3) {
+#pragma unroll
+                  for (int w = 0; w < 8; ++w) dc[w] += d2[w];
+                }
+              } else {
+                ptx::tmem_ld8(acc_base + 128 + ch * 8, dc);
+                ptx::tmem_wait_ld();
+              }
 #pragma unroll
               for (int w = 0; w < 8; ++w) R[q * 8 + w] += dm[w] + dc[w];
             }
@@ -1441,29 +1596,8 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_tc_grouped(const GrpArgs g) {
         ptx::tc_fence_after();
         const bool last = s_in == kc - 1 || s == it.nk - 1;
         if (ptx::elect_one()) {
-          const uint32_t acc_base = tmem + (uint32_t)((u & 1) * 256);
-          const uint32_t bb = smem_base + WS_OFF_BUF + b * BUF_BYTES;
-          const int ksteps = max(1, min(2, (it.K - s * TC_BK + 15) / 16));
-#pragma unroll
-          for (int ks = 0; ks < 2; ++ks) {
-            if (ks >= ksteps) break;
-            const uint32_t acc = (s_in > 0 || ks > 0) ? 1u : 0u;
-            uint64_t da[3], db[3];  // da: op(B) columns (MMA rows), db: A rows
-#pragma unroll
-            for (int sp = 0; sp < NSPLIT; ++sp) {
-              da[sp] = ptx::smem_desc(bb + sp * SPLIT_BYTES + 8192 + ks * 2 * CHUNK_BYTES,
-                                      CHUNK_BYTES, 128);
-              db[sp] = ptx::smem_desc(bb + sp * SPLIT_BYTES + ks * 2 * CHUNK_BYTES, CHUNK_BYTES, 128);
-            }
-            ptx::mma_bf16(acc_base, da[0], db[0], idesc, acc);
-            ptx::mma_bf16(acc_base + 128, da[0], db[1], idesc, acc);
-            ptx::mma_bf16(acc_base + 128, da[1], db[0], idesc, 1u);
-            if (NSPLIT == 3) {
-              ptx::mma_bf16(acc_base + 128, da[0], db[2], idesc, 1u);
-              ptx::mma_bf16(acc_base + 128, da[2], db[0], idesc, 1u);
-              ptx::mma_bf16(acc_base + 128, da[1], db[1], idesc, 1u);
-            }
-          }
+          tc_issue<NSPLIT, true, WsLayout<false>>(
+              b, (int)(u & 1), smem_base, idesc, s_in > 0 ? 1u : 0u, it.K - s * TC_BK > 16);
           ptx::mma_commit(&bars[B_BEMPTY + b]);
           if (last) ptx::mma_commit(&bars[B_AFULL + (u & 1)]);
         }
@@ -1871,7 +2005,7 @@ int tc_launch(TcProblem &p, int mode) {
     const bool wide = !drain && wa.c_tma;
     // long K on tiles of at most 64 columns: one 32-column block per epilogue
     // warp, a fold of 32 registers instead of 64 (no spills)
-    const bool narrow = drain && p.tile_n <= 32 * (WsRoles<false>::NE / 4);
+    const bool narrow = drain && p.tile_n <= 32 * (WsRoles<false, true>::NE / 4);
     const void *kern =
         mode == LIBSHALOM_PREC_BF16X6
             ? (narrow ? (const void *)k_tc_ws<3, true, false, 1>
@@ -1882,7 +2016,9 @@ int tc_launch(TcProblem &p, int mode) {
                : drain ? (const void *)k_tc_ws<2, true, false>
                : wide  ? (const void *)k_tc_ws<2, false, true>
                        : (const void *)k_tc_ws<2, false, false>);
-    const int threads = wide ? WsRoles<true>::THREADS : WsRoles<false>::THREADS;
+    const int threads = wide     ? WsRoles<true, false>::THREADS
+                        : narrow ? WsRoles<false, true>::THREADS
+                                 : WsRoles<false, false>::THREADS;
     (void)occupancy_of(kern, threads, WS_SMEM, 1);  // raises the shared-memory limit
     const int grid = grid_for(p.num_tiles, 1);
     void *args[] = {&ma, &mb, &mc, &wa};
