@@ -115,4 +115,35 @@ int finish_launch(const char *what);
 
 inline long cdiv(long a, long b) { return (a + b - 1) / b; }
 
+// Launch of a kernel that waits for its predecessor on the device
+// (chain_wait): its blocks are put in place while the predecessor runs.
+template <class... P, class... A>
+int launch_chained(void (*kern)(P...), long grid, int threads, size_t smem, cudaStream_t stream,
+                   A... args) {
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  LS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+  return LIBSHALOM_SUCCESS;
+}
+
+#ifdef __CUDACC__
+// First statement of every thread of a kernel launched with launch_chained:
+// the kernels before it have completed and their writes are visible, so that
+// nothing it does, or a kernel after it, can overtake them.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel's blocks take the places that are left (after this
+// kernel's own blocks have all been placed).
+__device__ __forceinline__ void chain_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 }  // namespace ls

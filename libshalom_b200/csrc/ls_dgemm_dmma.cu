@@ -5,8 +5,7 @@
 // whose C block fits a 32 x 32 warp tile.  One warp owns a run from its first
 // product to its last: the C block lives in the warp's registers as DMMA
 // accumulator fragments, so runs need no atomics and the result does not
-// depend on scheduling.  Runs are ordered heaviest first (counting sort on
-// their operand volume) and dealt round-robin to the warps of the grid.
+// depend on scheduling.  Runs are listed by shape and heaviest first, and dealt round-robin to the warps of the grid.
 //
 // Operands go from global memory straight into the fragments: a lane of
 // mma.sync.m8n8k4 holds A[lane / 4][lane % 4] and B[lane % 4][lane / 4], so a
@@ -23,9 +22,9 @@
 // Measured on 200,000 products with edges of 5 to 32 in runs of 8: 683 us when
 // the operands went through a ring of shared-memory slots (bulk copies, or
 // 16-byte cp.async for row windows; 280 M warp instructions, most of them
-// addresses and window shifts), 382 us now (130 M), of which the plan and the
-// CUDA-core kernel's look at its empty list are 32 us; the products' bytes
-// take 174 us.  8,000 products in runs of 8, 1,000 warps' work: 66 -> 52 us.
+// addresses and window shifts), 376 us now (130 M), of which the run list and
+// the CUDA-core kernel's look at its empty list are 25 us; the products' bytes
+// take 174 us.  8,000 products in runs of 8, 1,000 warps' work: 66 -> 42 us.
 // What is left is latency: the FP64 tensor pipe is 33-41 % busy and the issue
 // slots 30-40 %.  More warps an SM lose their cache lines to each other before
 // a line's second fragment is read (4 CTAs an SM, 32 x 32 blocks: 158 us
@@ -35,9 +34,8 @@
 // after the other: 406 us, and 111 us on the 8,000.
 #include <cuda_runtime.h>
 
-#include <algorithm>
-
 #include "ls_common.cuh"
+#include "ls_dgemm_runs.cuh"
 #include "ls_simt_launch.h"
 
 namespace ls {
@@ -47,104 +45,6 @@ namespace {
 constexpr int DM_WARPS = 4;     // warps per CTA (one run each at a time)
 constexpr int DM_KB = 3;        // k-steps of 4 loaded before they are multiplied
 constexpr int DM_PER_SM = 3;    // CTAs an SM holds (registers)
-constexpr int DM_CLASSES = 64;  // run cost classes of the heaviest-first order
-// Shapes of a run's C block, each with its own code (the loads and DMMAs issued
-// follow the fragments it may have; one code for all: 498 us): 0 both edges
-// above 16, 1 at most 16 columns, 2 at most 16 rows
-constexpr int DM_SHAPES = 3;
-constexpr int DM_BINS = DM_SHAPES * DM_CLASSES;
-
-struct DmPlan {
-  unsigned *n_large;
-  unsigned *n_shape, *shape_off;                  // [DM_SHAPES] runs, first slot
-  unsigned *bin_runs, *bin_off, *bin_fill;        // [DM_BINS] each
-  unsigned *small_first, *small_len;
-  unsigned *large_first, *large_len;
-};
-
-__device__ __forceinline__ bool dm_run_start(const LibShalom_dgemm_entry *e, long i) {
-  return i == 0 || e[i].C != e[i - 1].C;
-}
-
-// run starting at entry i: length, and its bin (shape, cost class: operand
-// doubles / 256, capped), or -1 for a C block that does not fit a warp tile
-__device__ __forceinline__ int dm_run_bin(const LibShalom_dgemm_entry *e, long count, long i,
-                                          long *len) {
-  const int M = e[i].M, N = e[i].N;
-  long cost = (long)M * N, j = i;
-  do {
-    const long K = max(0, e[j].K);
-    cost += K * (M + N);
-    ++j;
-  } while (j < count && e[j].C == e[i].C);
-  *len = j - i;
-  if (M > 32 || N > 32) return -1;
-  const int shape = M <= 16 ? 2 : N <= 16 ? 1 : 0;
-  return shape * DM_CLASSES + (int)max(0L, min(cost / 256, (long)DM_CLASSES - 1));
-}
-
-// Runs are counted per block in shared memory first: thousands of atomics on
-// a few words of global memory would take longer than the pass itself.
-__global__ void __launch_bounds__(256)
-    k_dm_count(const LibShalom_dgemm_entry *e, long count, DmPlan pl) {
-  __shared__ unsigned n[DM_BINS];
-  if (threadIdx.x < DM_BINS) n[threadIdx.x] = 0;
-  __syncthreads();
-  for (long i = blockIdx.x * 256L + threadIdx.x; i < count; i += gridDim.x * 256L) {
-    if (!dm_run_start(e, i)) continue;
-    long len;
-    const int bin = dm_run_bin(e, count, i, &len);
-    if (bin >= 0) {
-      atomicAdd(&n[bin], 1u);
-    } else {
-      const unsigned slot = atomicAdd(pl.n_large, 1u);
-      pl.large_first[slot] = (unsigned)i;
-      pl.large_len[slot] = (unsigned)len;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < DM_BINS && n[threadIdx.x])
-    atomicAdd(&pl.bin_runs[threadIdx.x], n[threadIdx.x]);
-}
-
-__global__ void __launch_bounds__(DM_BINS) k_dm_offsets(DmPlan pl) {
-  __shared__ unsigned n[DM_BINS];
-  const int b = threadIdx.x, shape = b / DM_CLASSES, lo = shape * DM_CLASSES;
-  n[b] = pl.bin_runs[b];
-  __syncthreads();
-  unsigned before = 0, in_shape = 0;
-  for (int i = 0; i < lo; ++i) before += n[i];
-  if (b == lo) pl.shape_off[shape] = before;
-  for (int i = lo + DM_CLASSES - 1; i > b; --i) in_shape += n[i];
-  pl.bin_off[b] = before + in_shape;
-  if (b == lo) pl.n_shape[shape] = in_shape + n[b];
-}
-
-__global__ void __launch_bounds__(256)
-    k_dm_place(const LibShalom_dgemm_entry *e, long count, DmPlan pl) {
-  __shared__ unsigned n[DM_BINS], base[DM_BINS];
-  for (long i0 = blockIdx.x * 256L; i0 < count; i0 += gridDim.x * 256L) {
-    if (threadIdx.x < DM_BINS) n[threadIdx.x] = 0;
-    __syncthreads();
-    const long i = i0 + threadIdx.x;
-    long len = 0;
-    int bin = -1;
-    unsigned rank = 0;
-    if (i < count && dm_run_start(e, i)) bin = dm_run_bin(e, count, i, &len);
-    if (bin >= 0) rank = atomicAdd(&n[bin], 1u);
-    __syncthreads();
-    if (threadIdx.x < DM_BINS && n[threadIdx.x])
-      base[threadIdx.x] = atomicAdd(&pl.bin_fill[threadIdx.x], n[threadIdx.x]);
-    __syncthreads();
-    if (bin >= 0) {
-      const unsigned slot = pl.bin_off[bin] + base[bin] + rank;
-      pl.small_first[slot] = (unsigned)i;
-      pl.small_len[slot] = (unsigned)len;
-    }
-    __syncthreads();
-  }
-}
-
 // predicated (warp-uniformly): a branch around each would multiply the live
 // ranges of the accumulators (1.1 KB of spills)
 __device__ __forceinline__ void dmma_if(double &d0, double &d1, double a, double b, bool on) {
@@ -244,12 +144,6 @@ struct DmWarp {
   uint32_t w;           // word `lane` of its first entry
 };
 
-// word `lane` of an entry: loaded a product ahead and broadcast when it is
-// needed, so that no product waits for its entry
-__device__ __forceinline__ uint32_t dm_word(const LibShalom_dgemm_entry *e, int lane) {
-  return lane < 18 ? reinterpret_cast<const uint32_t *>(e)[lane] : 0u;
-}
-
 // the warp's runs below `end`, of C blocks within FM x FN fragments
 template <int FM, int FN>
 __device__ __forceinline__ void dm_runs(DmWarp &s, long end, int lane) {
@@ -288,7 +182,7 @@ __device__ __forceinline__ void dm_runs(DmWarp &s, long end, int lane) {
                 ldb = (int)get(11);
       const double alpha = __longlong_as_double((long long)get64(14));
       const double beta = __longlong_as_double((long long)get64(16));
-      if (p + 1 < n || more) s.w = dm_word(s.entries + (p + 1 < n ? at + p + 1 : s.first), lane);
+      if (p + 1 < n || more) s.w = entry_word(s.entries + (p + 1 < n ? at + p + 1 : s.first), lane);
       if (beta == 0.0) {
 #pragma unroll
         for (int mf = 0; mf < FM; ++mf)
@@ -320,7 +214,9 @@ __device__ __forceinline__ void dm_runs(DmWarp &s, long end, int lane) {
 }
 
 __global__ void __launch_bounds__(DM_WARPS * 32, DM_PER_SM)
-    k_dgemm_dmma(const LibShalom_dgemm_entry *entries, const DmPlan pl) {
+    k_dgemm_dmma(const LibShalom_dgemm_entry *entries, const RunPlan pl) {
+  chain_wait();
+  chain_next();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long end0 = pl.n_shape[0], end1 = end0 + pl.n_shape[1], end2 = end1 + pl.n_shape[2];
   DmWarp s;
@@ -333,7 +229,7 @@ __global__ void __launch_bounds__(DM_WARPS * 32, DM_PER_SM)
   if (s.r >= s.n_runs) return;
   s.first = s.run_first[s.r];
   s.len = s.run_len[s.r];
-  s.w = dm_word(entries + s.first, lane);
+  s.w = entry_word(entries + s.first, lane);
   dm_runs<4, 4>(s, end0, lane);
   dm_runs<4, 2>(s, end1, lane);
   dm_runs<2, 4>(s, end2, lane);
@@ -342,35 +238,13 @@ __global__ void __launch_bounds__(DM_WARPS * 32, DM_PER_SM)
 }  // namespace
 
 int run_dgemm_dmma(const LibShalom_dgemm_entry *entries, long count) {
-  State &st = state();
-  if (count > (1L << 30)) return LIBSHALOM_ERR_UNSUPPORTED;
-  void *ws = nullptr;
-  const size_t header = 1024;
-  const size_t words = header + 4 * (size_t)count;
-  int rc = workspace(words * sizeof(unsigned), &ws);
+  RunPlan pl;
+  int rc = plan_dgemm_runs(entries, count, &pl);
   if (rc) return rc;
-  unsigned *w = static_cast<unsigned *>(ws);
-  DmPlan pl;
-  pl.n_large = w;
-  pl.n_shape = w + 8;
-  pl.shape_off = w + 16;
-  pl.bin_runs = w + 64;
-  pl.bin_off = pl.bin_runs + DM_BINS;
-  pl.bin_fill = pl.bin_off + DM_BINS;
-  pl.small_first = w + header;
-  pl.small_len = pl.small_first + count;
-  pl.large_first = pl.small_len + count;
-  pl.large_len = pl.large_first + count;
-  LS_CUDA_TRY(cudaMemsetAsync(w, 0, header * sizeof(unsigned), st.stream));
-  const int pgrid = (int)std::max(1L, std::min(cdiv(count, 256), (long)st.num_sms * 8));
-  k_dm_count<<<pgrid, 256, 0, st.stream>>>(entries, count, pl);
-  k_dm_offsets<<<1, DM_BINS, 0, st.stream>>>(pl);
-  k_dm_place<<<pgrid, 256, 0, st.stream>>>(entries, count, pl);
-  LS_CUDA_TRY(cudaGetLastError());
   const int per_sm = occupancy_of((const void *)k_dgemm_dmma, DM_WARPS * 32, 0, DM_PER_SM);
-  k_dgemm_dmma<<<grid_for(cdiv(count, DM_WARPS), per_sm), DM_WARPS * 32, 0, st.stream>>>(entries,
-                                                                                        pl);
-  LS_CUDA_TRY(cudaGetLastError());
+  rc = launch_chained(k_dgemm_dmma, grid_for(cdiv(count, DM_WARPS), per_sm), DM_WARPS * 32, 0,
+                      state().stream, entries, pl);
+  if (rc) return rc;
   return run_dgemm_runs_list(entries, count, pl.n_large, pl.large_first, pl.large_len);
 }
 

@@ -32,7 +32,7 @@ int run_grouped_d(const LibShalom_dgemm_entry *entries, long count);
 // C = alpha * sum_z partial[z] + beta * C, partial slices summed in order
 int run_splitk_reduce_f32(const float *partial, int splits, long M, long N, float *C, long ldc,
                           float alpha, float beta);
-// ls_dgemm.cu: runs of products sharing C, C tile held in registers
+// ls_dgemm.cu: runs of products sharing C, the C block held in registers
 int run_dgemm_runs(const LibShalom_dgemm_entry *entries, long count);
 int run_dgemm_runs_list(const LibShalom_dgemm_entry *entries, long count, const unsigned *n_runs,
                         const unsigned *run_first, const unsigned *run_len);
@@ -40,7 +40,7 @@ int run_dgemm_runs_list(const LibShalom_dgemm_entry *entries, long count, const 
 // tensor cores, the rest through run_dgemm_runs_list
 int run_dgemm_warp(const LibShalom_dgemm_entry *entries, long count, int method, int slices);
 // ls_dgemm_dmma.cu: runs with M, N <= 32 on the FP64 tensor cores (warp per
-// run, bulk-copy ring), the rest through run_dgemm_runs_list
+// run), the rest through run_dgemm_runs_list
 int run_dgemm_dmma(const LibShalom_dgemm_entry *entries, long count);
 
 // Plain FP32 split-K GEMM (GEMM_K-aligned slices, rounding order of the mp
