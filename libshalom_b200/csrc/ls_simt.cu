@@ -23,6 +23,7 @@ k_gemm_single(GemmArgs<T> g, int tiles_m, int tiles_n, int ways_m, int ways_n,
               int splits, long kchunk, T *partial) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *smem = reinterpret_cast<T *>(smem_raw);
+  if (splits > 1) chain_next();
   // Work item -> (k slice z, tile row tm, tile column tn).  Without a ways
   // partition a work item is one tile.  With LibShalom_set_thread_ways the
   // tile grid is cut into ways_m x ways_n rectangular groups and a work item
@@ -61,6 +62,7 @@ k_gemm_single(GemmArgs<T> g, int tiles_m, int tiles_n, int ways_m, int ways_n,
 template <typename T>
 __global__ void k_splitk_reduce(const T *partial, int splits, long M, long N,
                                 T *C, long ldc, T alpha, T beta) {
+  chain_wait();
   const long total = M * N;
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total;
        e += (long)gridDim.x * blockDim.x) {
@@ -258,6 +260,15 @@ struct Dispatch<double> {
 };
 
 template <typename T>
+static int launch_reduce(const T *partial, int splits, long M, long N, T *C, long ldc, T alpha,
+                         T beta) {
+  State &st = state();
+  const long grid = std::max(1L, std::min(cdiv(M * N, 256), (long)st.num_sms * 8));
+  return launch_chained(k_splitk_reduce<T>, grid, 256, 0, st.stream, partial, splits, M, N, C, ldc,
+                        alpha, beta);
+}
+
+template <typename T>
 int run_gemm(const GemmArgs<T> &g, const SimtOptions &opt, SimtPlan *plan_out) {
   State &st = state();
   int ncfg;
@@ -293,13 +304,8 @@ int run_gemm(const GemmArgs<T> &g, const SimtOptions &opt, SimtPlan *plan_out) {
   int rc = Dispatch<T>::single(cfg, g, splits, kchunk, partial, opt.ways_m, opt.ways_n,
                                opt.kblock);
   if (rc) return rc;
-  if (splits > 1) {
-    const long total = g.M * g.N;
-    int grid = (int)std::min<long>(cdiv(total, 256), (long)st.num_sms * 8);
-    k_splitk_reduce<T><<<std::max(grid, 1), 256, 0, st.stream>>>(partial, splits, g.M, g.N,
-                                                                g.C, g.ldc, g.alpha, g.beta);
-    LS_CUDA_TRY(cudaGetLastError());
-  }
+  if (splits > 1)
+    return launch_reduce<T>(partial, splits, g.M, g.N, g.C, g.ldc, g.alpha, g.beta);
   return LIBSHALOM_SUCCESS;
 }
 
@@ -316,23 +322,12 @@ int run_gemm_splitk_external(const GemmArgs<float> &g, int splits, float *partia
   const int used = g.K > 0 ? (int)cdiv(g.K, kchunk) : 1;
   int rc = Dispatch<float>::single(cfg, g, used, kchunk, partial, 0, 0, true);
   if (rc || used == 1) return rc;  // one slice: the tile kernel wrote C itself
-  const long total = g.M * g.N;
-  const int grid = (int)std::min<long>(cdiv(total, 256), (long)st.num_sms * 8);
-  k_splitk_reduce<float><<<std::max(grid, 1), 256, 0, st.stream>>>(partial, used, g.M, g.N,
-                                                                  g.C, g.ldc, g.alpha, g.beta);
-  LS_CUDA_TRY(cudaGetLastError());
-  return LIBSHALOM_SUCCESS;
+  return launch_reduce<float>(partial, used, g.M, g.N, g.C, g.ldc, g.alpha, g.beta);
 }
 
 int run_splitk_reduce_f32(const float *partial, int splits, long M, long N, float *C, long ldc,
                           float alpha, float beta) {
-  State &st = state();
-  const long total = M * N;
-  const int grid = (int)std::min<long>(cdiv(total, 256), (long)st.num_sms * 8);
-  k_splitk_reduce<float><<<std::max(grid, 1), 256, 0, st.stream>>>(partial, splits, M, N, C, ldc,
-                                                                  alpha, beta);
-  LS_CUDA_TRY(cudaGetLastError());
-  return LIBSHALOM_SUCCESS;
+  return launch_reduce<float>(partial, splits, M, N, C, ldc, alpha, beta);
 }
 
 template int run_gemm<float>(const GemmArgs<float> &, const SimtOptions &, SimtPlan *);
