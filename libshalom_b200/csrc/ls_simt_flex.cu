@@ -53,16 +53,22 @@ __global__ void __launch_bounds__(FX_THREADS, PER_SM) k_flex_uniform(const FlexU
 // ---------------------------------------------------------------------------
 constexpr int FG_CLASSES = 64;  // work classes: half octaves of M N K a part
 constexpr int FG_PARTS = 16;    // a run's tiles are dealt to at most 16 items
+// Wide items a CTA up to which the small list's blocks start beside the wide
+// list's: their tails fill each other, but the two share an SM's L1 from then
+// on.  Mixed batches of 4..256, beside against behind: 50 products 52 (84) us,
+// 1,000 116 (157), 5,000 244 (338), 20,000 654 (659), 35,000 1,111 (1,066),
+// 50,000 1,548 (1,488).
+constexpr unsigned FG_BESIDE = 20;
 constexpr unsigned FG_LONG = (1u << 28) - 1;  // products of a run an item word can hold
 
 // Plan: every run of entries sharing C becomes min(tiles, parts) items {first
 // entry, products << 4 | part}, counting-sorted heaviest first, in two lists:
 // C of more than 64 columns and 32 rows takes 64 x 128 tiles of 8 x 8 outputs
 // a thread, the rest 64 x 64 tiles of 8 x 4 or 4 x 4 (one list for all: 1.57 ms
-// on 50,000 products of 4..256, two lists 1.51 ms; one CTA a run on 64 x 64
+// on 50,000 products of 4..256, two lists 1.49 ms; one CTA a run on 64 x 64
 // tiles, as before: 4.66 ms).  The lists fill one array from its two ends.
 struct FlexPlan {
-  unsigned *class_n, *class_off, *class_fill;  // [2][FG_CLASSES]: small, wide
+  unsigned *class_n, *class_fill;  // [2][FG_CLASSES]: small, wide
   unsigned *n_items, *counter;                 // [2]
   uint2 *items;  // [n]: small ones upwards from 0, wide ones downwards from n - 1
   long n;        // parts * count
@@ -96,42 +102,62 @@ __device__ __forceinline__ int fg_run(const LibShalom_sgemm_entry *e, long count
   return parts;
 }
 
-__global__ void k_fg_count(const LibShalom_sgemm_entry *e, long count, FlexPlan pl) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count;
-       i += (long)gridDim.x * blockDim.x) {
-    if (i > 0 && e[i].C == e[i - 1].C) continue;
-    long len;
-    int cls;
-    const int parts = fg_run(e, count, i, pl.parts, &len, &cls);
-    if (parts) atomicAdd(&pl.class_n[cls], (unsigned)parts);
-  }
-}
-
-__global__ void __launch_bounds__(2 * FG_CLASSES) k_fg_offsets(FlexPlan pl) {
+// Items are counted per block in shared memory first: a call's atomics on the
+// few words of the classes took 17 us on 50,000 products.
+__global__ void __launch_bounds__(256)
+    k_fg_count(const LibShalom_sgemm_entry *e, long count, FlexPlan pl) {
   __shared__ unsigned n[2 * FG_CLASSES];
-  const int c = threadIdx.x, list = c / FG_CLASSES, lo = list * FG_CLASSES;
-  n[c] = pl.class_n[c];
+  chain_next();
+  if (threadIdx.x < 2 * FG_CLASSES) n[threadIdx.x] = 0;
   __syncthreads();
-  unsigned before = 0;
-  for (int i = lo + FG_CLASSES - 1; i > c; --i) before += n[i];
-  pl.class_off[c] = before;
-  if (c == lo) pl.n_items[list] = before + n[c];
-}
-
-__global__ void k_fg_place(const LibShalom_sgemm_entry *e, long count, FlexPlan pl) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count;
-       i += (long)gridDim.x * blockDim.x) {
+  for (long i = blockIdx.x * 256L + threadIdx.x; i < count; i += gridDim.x * 256L) {
     if (i > 0 && e[i].C == e[i - 1].C) continue;
     long len;
     int cls;
     const int parts = fg_run(e, count, i, pl.parts, &len, &cls);
-    if (!parts) continue;
-    const unsigned slot = pl.class_off[cls] + atomicAdd(&pl.class_fill[cls], (unsigned)parts);
-    const unsigned n = (unsigned)min(len, (long)FG_LONG);
+    if (parts) atomicAdd(&n[cls], (unsigned)parts);
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 * FG_CLASSES && n[threadIdx.x])
+    atomicAdd(&pl.class_n[threadIdx.x], n[threadIdx.x]);
+}
+
+// Every block sums the classes itself: heavy classes of a list come first.
+__global__ void __launch_bounds__(256)
+    k_fg_place(const LibShalom_sgemm_entry *e, long count, FlexPlan pl) {
+  __shared__ unsigned all[2 * FG_CLASSES], off[2 * FG_CLASSES], n[2 * FG_CLASSES],
+      base[2 * FG_CLASSES];
+  chain_wait();
+  chain_next();
+  const int tid = threadIdx.x;
+  if (tid < 2 * FG_CLASSES) all[tid] = pl.class_n[tid];
+  __syncthreads();
+  if (tid < 2 * FG_CLASSES) {
+    const int lo = tid & ~(FG_CLASSES - 1);
+    unsigned before = 0;
+    for (int i = lo + FG_CLASSES - 1; i > tid; --i) before += all[i];
+    off[tid] = before;
+    if (blockIdx.x == 0 && tid == lo) pl.n_items[lo / FG_CLASSES] = before + all[tid];
+  }
+  for (long i0 = blockIdx.x * 256L; i0 < count; i0 += gridDim.x * 256L) {
+    if (tid < 2 * FG_CLASSES) n[tid] = 0;
+    __syncthreads();
+    const long i = i0 + tid;
+    long len = 0;
+    int cls = 0, parts = 0;
+    if (i < count && (i == 0 || e[i].C != e[i - 1].C))
+      parts = fg_run(e, count, i, pl.parts, &len, &cls);
+    const unsigned rank = parts ? atomicAdd(&n[cls], (unsigned)parts) : 0;
+    __syncthreads();
+    if (tid < 2 * FG_CLASSES && n[tid]) base[tid] = atomicAdd(&pl.class_fill[tid], n[tid]);
+    __syncthreads();
+    const unsigned products = (unsigned)min(len, (long)FG_LONG);
     for (int p = 0; p < parts; ++p) {
-      const long at = (long)slot + p;
-      pl.items[cls < FG_CLASSES ? at : pl.n - 1 - at] = make_uint2((unsigned)i, n << 4 | (unsigned)p);
+      const long at = (long)off[cls] + base[cls] + rank + p;
+      pl.items[cls < FG_CLASSES ? at : pl.n - 1 - at] =
+          make_uint2((unsigned)i, products << 4 | (unsigned)p);
     }
+    __syncthreads();
   }
 }
 
@@ -144,7 +170,12 @@ __global__ void __launch_bounds__(FX_THREADS, WIDE ? 4 : 6)
     k_flex_grouped(const LibShalom_sgemm_entry *entries, long count, FlexPlan pl) {
   extern __shared__ __align__(16) float fsm[];
   __shared__ uint2 s_item[2];
+  if constexpr (WIDE) chain_wait();  // the plan
   const unsigned n_items = pl.n_items[WIDE];
+  // The small list's blocks may start when all of this kernel's have: the plan
+  // is complete then, nothing that either writes is the other's, and the wait
+  // at the end keeps what follows in the stream behind both.
+  if (WIDE && n_items <= FG_BESIDE * gridDim.x) chain_next();
   uint2 nxt = make_uint2(0, 0);
   unsigned idx = 0;
   auto take = [&]() {
@@ -201,6 +232,7 @@ __global__ void __launch_bounds__(FX_THREADS, WIDE ? 4 : 6)
     }
     __syncthreads();
   }
+  if constexpr (!WIDE) chain_wait();
 }
 
 template <class Cfg, int TM, int TN, int PER_SM>
@@ -257,24 +289,23 @@ int run_grouped_s(const LibShalom_sgemm_entry *entries, long count) {
   unsigned *w = static_cast<unsigned *>(ws);
   pl.n = pl.parts * count;
   pl.class_n = w;
-  pl.class_off = w + 2 * FG_CLASSES;
-  pl.class_fill = w + 4 * FG_CLASSES;
-  pl.n_items = w + 6 * FG_CLASSES;
+  pl.class_fill = w + 2 * FG_CLASSES;
+  pl.n_items = w + 4 * FG_CLASSES;
   pl.counter = pl.n_items + 2;
   pl.items = reinterpret_cast<uint2 *>(w + header);
   LS_CUDA_TRY(cudaMemsetAsync(w, 0, header * sizeof(unsigned), st.stream));
   const int pgrid = (int)std::max(1L, std::min(cdiv(count, 256), (long)st.num_sms * 8));
   k_fg_count<<<pgrid, 256, 0, st.stream>>>(entries, count, pl);
-  k_fg_offsets<<<1, 2 * FG_CLASSES, 0, st.stream>>>(pl);
-  k_fg_place<<<pgrid, 256, 0, st.stream>>>(entries, count, pl);
   LS_CUDA_TRY(cudaGetLastError());
+  if ((rc = launch_chained(k_fg_place, pgrid, 256, 0, st.stream, entries, count, pl))) return rc;
   const int ps_w = occupancy_of((const void *)k_flex_grouped<true>, FX_THREADS, F128::SMEM, 4);
   const int ps_s = occupancy_of((const void *)k_flex_grouped<false>, FX_THREADS, F64::SMEM, 6);
-  k_flex_grouped<true><<<grid_for((long)st.num_sms * ps_w, ps_w), FX_THREADS, F128::SMEM,
-                         st.stream>>>(entries, count, pl);
-  k_flex_grouped<false><<<grid_for((long)st.num_sms * ps_s, ps_s), FX_THREADS, F64::SMEM,
-                          st.stream>>>(entries, count, pl);
-  LS_CUDA_TRY(cudaGetLastError());
+  rc = launch_chained(k_flex_grouped<true>, grid_for((long)st.num_sms * ps_w, ps_w), FX_THREADS,
+                      F128::SMEM, st.stream, entries, count, pl);
+  if (rc) return rc;
+  rc = launch_chained(k_flex_grouped<false>, grid_for((long)st.num_sms * ps_s, ps_s), FX_THREADS,
+                      F64::SMEM, st.stream, entries, count, pl);
+  if (rc) return rc;
   return LIBSHALOM_SUCCESS;
 }
 

@@ -1265,20 +1265,29 @@ __device__ __forceinline__ int grp_run_class(const LibShalom_sgemm_entry *e, lon
 }
 
 // pass 1: items per work class
-__global__ void k_grp_count(const LibShalom_sgemm_entry *e, long count, GrpPlan pl) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count;
-       i += (long)gridDim.x * blockDim.x) {
+// (counted per block in shared memory first: a call's atomics on the few words
+// of the classes took 17 us on 50,000 products)
+__global__ void __launch_bounds__(256)
+    k_grp_count(const LibShalom_sgemm_entry *e, long count, GrpPlan pl) {
+  static_assert(4 * GRP_CLASSES == 256, "one thread a class");
+  __shared__ unsigned n[4 * GRP_CLASSES];
+  chain_next();
+  n[threadIdx.x] = 0;
+  __syncthreads();
+  for (long i = blockIdx.x * 256L + threadIdx.x; i < count; i += gridDim.x * 256L) {
     if (!grp_run_start(e, i)) continue;
     long len;
     int kind, tiles;
     const int cls = grp_run_class(e, count, i, pl.items != nullptr, &len, &kind, &tiles);
-    if (kind == GRP_SMALL) atomicAdd(&pl.class_n[cls], (unsigned)tiles);
-    if (kind == GRP_LARGE) atomicAdd(&pl.class_n[GRP_CLASSES + cls], 1u);
+    if (kind == GRP_SMALL) atomicAdd(&n[cls], (unsigned)tiles);
+    if (kind == GRP_LARGE) atomicAdd(&n[GRP_CLASSES + cls], 1u);
     if (kind == GRP_EITHER) {
-      atomicAdd(&pl.class_n[2 * GRP_CLASSES + cls], (unsigned)tiles);
-      atomicAdd(&pl.class_n[3 * GRP_CLASSES + cls], 1u);
+      atomicAdd(&n[2 * GRP_CLASSES + cls], (unsigned)tiles);
+      atomicAdd(&n[3 * GRP_CLASSES + cls], 1u);
     }
   }
+  __syncthreads();
+  if (n[threadIdx.x]) atomicAdd(&pl.class_n[threadIdx.x], n[threadIdx.x]);
 }
 
 // pass 2: first sorted slot of every class, heaviest class first (one block of
@@ -1286,6 +1295,8 @@ __global__ void k_grp_count(const LibShalom_sgemm_entry *e, long count, GrpPlan 
 __global__ void __launch_bounds__(GRP_CLASSES) k_grp_offsets(GrpPlan pl) {
   __shared__ unsigned n[4][GRP_CLASSES];
   __shared__ int s_large;
+  chain_wait();
+  chain_next();
   const int c = threadIdx.x;
   for (int k = 0; k < 4; ++k) n[k][c] = pl.class_n[k * GRP_CLASSES + c];
   __syncthreads();
@@ -1312,26 +1323,36 @@ __global__ void __launch_bounds__(GRP_CLASSES) k_grp_offsets(GrpPlan pl) {
 }
 
 // pass 3: every item takes a slot in its class's range
-__global__ void k_grp_place(const LibShalom_sgemm_entry *e, long count, GrpPlan pl) {
+__global__ void __launch_bounds__(256)
+    k_grp_place(const LibShalom_sgemm_entry *e, long count, GrpPlan pl) {
+  __shared__ unsigned n[2 * GRP_CLASSES], base[2 * GRP_CLASSES];
+  chain_wait();
+  chain_next();
   const bool either_large = *pl.either_large != 0;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count;
-       i += (long)gridDim.x * blockDim.x) {
-    if (!grp_run_start(e, i)) continue;
-    long len;
-    int kind, tiles;
-    int cls = grp_run_class(e, count, i, pl.items != nullptr, &len, &kind, &tiles);
-    if (kind == GRP_EMPTY) continue;
+  const int tid = threadIdx.x;
+  for (long i0 = blockIdx.x * 256L; i0 < count; i0 += gridDim.x * 256L) {
+    if (tid < 2 * GRP_CLASSES) n[tid] = 0;
+    __syncthreads();
+    const long i = i0 + tid;
+    long len = 0;
+    int kind = GRP_EMPTY, tiles = 0, cls = 0;
+    if (i < count && grp_run_start(e, i))
+      cls = grp_run_class(e, count, i, pl.items != nullptr, &len, &kind, &tiles);
     const bool large = kind == GRP_LARGE || (kind == GRP_EITHER && either_large);
     if (large) cls += GRP_CLASSES;
-    const unsigned slot =
-        pl.class_off[cls] + atomicAdd(&pl.class_fill[cls], large ? 1u : (unsigned)tiles);
+    const unsigned rank = kind == GRP_EMPTY ? 0 : atomicAdd(&n[cls], large ? 1u : (unsigned)tiles);
+    __syncthreads();
+    if (tid < 2 * GRP_CLASSES && n[tid])
+      base[tid] = pl.class_off[tid] + atomicAdd(&pl.class_fill[tid], n[tid]);
+    __syncthreads();
     if (large) {
-      pl.run_first[slot] = (unsigned)i;
-      pl.run_len[slot] = (unsigned)len;
-    } else {
+      pl.run_first[base[cls] + rank] = (unsigned)i;
+      pl.run_len[base[cls] + rank] = (unsigned)len;
+    } else if (kind != GRP_EMPTY) {
       for (int t = 0; t < tiles; ++t)
-        pl.items[slot + t] = make_uint2((unsigned)i, (unsigned)len << 3 | (unsigned)t);
+        pl.items[base[cls] + rank + t] = make_uint2((unsigned)i, (unsigned)len << 3 | (unsigned)t);
     }
+    __syncthreads();
   }
 }
 
@@ -1452,6 +1473,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_tc_grouped(const GrpArgs g) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t smem_base = ptx::smem_u32(smem);
   const int kc = g.kc_slabs;
+  chain_wait();
   if (*g.n_runs == 0) return;  // every run went to the small-product kernel
 
   if (tid == 0) {
@@ -2196,9 +2218,10 @@ int tc_sgemm_grouped(const LibShalom_sgemm_entry *entries, long count, int mode)
   LS_CUDA_TRY(cudaMemsetAsync(w, 0, GRP_HEADER * sizeof(unsigned), st.stream));
   const int pgrid = (int)std::max(1L, std::min(cdiv(count, 256), (long)st.num_sms * 8));
   k_grp_count<<<pgrid, 256, 0, st.stream>>>(entries, count, pl);
-  k_grp_offsets<<<1, GRP_CLASSES, 0, st.stream>>>(pl);
-  k_grp_place<<<pgrid, 256, 0, st.stream>>>(entries, count, pl);
   LS_CUDA_TRY(cudaGetLastError());
+  int rc = launch_chained(k_grp_offsets, 1, GRP_CLASSES, 0, st.stream, pl);
+  if (!rc) rc = launch_chained(k_grp_place, pgrid, 256, 0, st.stream, entries, count, pl);
+  if (rc) return rc;
 
   void *errp = nullptr;
   LS_CUDA_TRY(cudaGetSymbolAddress(&errp, g_tc_err));
@@ -2209,7 +2232,7 @@ int tc_sgemm_grouped(const LibShalom_sgemm_entry *entries, long count, int mode)
     sa.n_items_dev = pl.n_items;
     sa.counter = pl.counter;
     sa.err = reinterpret_cast<unsigned *>(errp);
-    const int rc = tc_small_launch(sa, false, mode);
+    rc = tc_small_launch(sa, false, mode);
     if (rc) return rc;
   }
   GrpArgs g;
@@ -2220,13 +2243,10 @@ int tc_sgemm_grouped(const LibShalom_sgemm_entry *entries, long count, int mode)
   g.n_runs = pl.n_items + 1;
   g.err = reinterpret_cast<unsigned *>(errp);
   g.kc_slabs = 128 / TC_BK;
-  const void *kern = mode == LIBSHALOM_PREC_BF16X6 ? (const void *)k_tc_grouped<3>
-                                                   : (const void *)k_tc_grouped<2>;
-  (void)occupancy_of(kern, G_THREADS, G_SMEM, 1);  // raises the shared-memory limit
-  const int grid = grid_for((long)st.num_sms, 1);
-  void *args[] = {&g};
-  LS_CUDA_TRY(cudaLaunchKernel(kern, dim3(grid), dim3(G_THREADS), args, G_SMEM, st.stream));
-  LS_CUDA_TRY(cudaGetLastError());
+  auto kern = mode == LIBSHALOM_PREC_BF16X6 ? k_tc_grouped<3> : k_tc_grouped<2>;
+  (void)occupancy_of((const void *)kern, G_THREADS, G_SMEM, 1);  // raises the shared-memory limit
+  rc = launch_chained(kern, grid_for((long)st.num_sms, 1), G_THREADS, G_SMEM, st.stream, g);
+  if (rc) return rc;
   if (st.sync) {
     unsigned err = 0;
     LS_CUDA_TRY(cudaStreamSynchronize(st.stream));

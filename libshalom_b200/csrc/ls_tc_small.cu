@@ -26,7 +26,7 @@
 // products of a chunk are issued in the order of the other split-BF16 kernels.
 //
 // Measured on a B200: 50,000 products of 4..256 (log-uniform, one in five
-// adding to its predecessor's C) 1.14 ms, against 2.66 ms with k_tc_grouped
+// adding to its predecessor's C) 1.11 ms, against 2.66 ms with k_tc_grouped
 // alone; 10,000 products of 45 x 37 x 51 96 us, against 465 us with
 // k_tc_sgemm.  Bound by instruction issue and latency (ncu, the mixed batch:
 // 55-60 % fewer warp instructions than k_tc_grouped, issue slots 47 % busy,
@@ -88,6 +88,10 @@ __device__ __forceinline__ unsigned fetch_inc(unsigned *p) {
 template <int NSPLIT, bool UNIFORM>
 __global__ void __launch_bounds__(SM_THREADS, SM_PER_SM) k_tc_small(const TcSmallArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
+  if constexpr (!UNIFORM) {  // the plan
+    chain_wait();
+    chain_next();
+  }
   // no static shared memory: it would move the operands off their alignment
   SmallSlot *slots = reinterpret_cast<SmallSlot *>(smem + SM_OFF_CTL);
   uint64_t &bar = *reinterpret_cast<uint64_t *>(smem + SM_OFF_CTL + 2 * sizeof(SmallSlot));
@@ -400,14 +404,12 @@ __global__ void __launch_bounds__(SM_THREADS, SM_PER_SM) k_tc_small(const TcSmal
 int tc_small_launch(const TcSmallArgs &a, bool uniform, int mode) {
   State &st = state();
   const bool x6 = mode == LIBSHALOM_PREC_BF16X6;
-  const void *kern = uniform ? (x6 ? (const void *)k_tc_small<3, true> : (const void *)k_tc_small<2, true>)
-                             : (x6 ? (const void *)k_tc_small<3, false>
-                                   : (const void *)k_tc_small<2, false>);
-  (void)occupancy_of(kern, SM_THREADS, SM_BYTES, SM_PER_SM);
+  auto kern = uniform ? (x6 ? k_tc_small<3, true> : k_tc_small<2, true>)
+                      : (x6 ? k_tc_small<3, false> : k_tc_small<2, false>);
+  (void)occupancy_of((const void *)kern, SM_THREADS, SM_BYTES, SM_PER_SM);
   const int grid = grid_for(uniform ? a.n_items : (long)st.num_sms * SM_PER_SM, SM_PER_SM);
-  TcSmallArgs args = a;
-  void *argv[] = {&args};
-  LS_CUDA_TRY(cudaLaunchKernel(kern, dim3(grid), dim3(SM_THREADS), argv, SM_BYTES, st.stream));
+  if (!uniform) return launch_chained(kern, grid, SM_THREADS, SM_BYTES, st.stream, a);
+  kern<<<grid, SM_THREADS, SM_BYTES, st.stream>>>(a);
   LS_CUDA_TRY(cudaGetLastError());
   return LIBSHALOM_SUCCESS;
 }
