@@ -738,7 +738,7 @@ def measure_mixed(args, torch, ls, s, count=50_000, cpu=True):
            "roofline": _roofline(alg_bytes, modes[best]["ms"], "sgemm grouped (bf16x6)"),
            "clocks": modes[best]["clocks"], "modes": modes, "per_call_fp32": per_call,
            "speedup_vs_per_call": modes[best]["gflops"] / per_call["gflops"],
-           "gpu_launches_per_step": 4}
+           "gpu_launches_per_step": 5}
     if cpu:
         from oracle import oracle as orc
         threads = orc.max_threads()
@@ -864,7 +864,7 @@ def measure_dgemm_runs(args, torch, ls, s, count=200_000, run=8, cpu=True):
            "roofline": _roofline(alg_bytes, methods[best]["ms"], f"dgemm grouped ({best})"),
            "clocks": methods[best]["clocks"], "methods": methods,
            "per_call_fp64": per_call, "speedup_vs_per_call": value / per_call["gflops"],
-           "gpu_launches_per_step": 2}
+           "gpu_launches_per_step": 4}
     if cpu:
         from oracle import oracle as orc
         threads = orc.max_threads()

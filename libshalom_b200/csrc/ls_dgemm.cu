@@ -26,8 +26,8 @@
 // 54.6 -> 48.2 us, the latency of a chain of loads; 8 k at a time made that 60.
 // 16 products: 12.3 -> 10.2 us (14.3 before each kernel's blocks were placed
 // while the one before runs).
-// The shared-memory pipe bounds it (wavefronts 70 % of its peak, FP64 pipe
-// 23 %): a lane's outputs lie 4 or 8 apart, so that the 8-byte loads of a warp
+// The shared-memory pipe bounds it (wavefronts 58 % of its peak, FP64 pipe
+// 25 %): a lane's outputs lie 4 or 8 apart, so that the 8-byte loads of a warp
 // read 4 to 8 neighbouring words; 4 x 4 neighbours with 16-byte loads took 594.
 // 4 CTAs an SM (spills, 8 k at a time) 618; 2 CTAs 601.
 //

@@ -22,11 +22,11 @@
 // Measured on 200,000 products with edges of 5 to 32 in runs of 8: 683 us when
 // the operands went through a ring of shared-memory slots (bulk copies, or
 // 16-byte cp.async for row windows; 280 M warp instructions, most of them
-// addresses and window shifts), 376 us now (130 M), of which the run list and
+// addresses and window shifts), 373 us now (142 M), of which the run list and
 // the CUDA-core kernel's look at its empty list are 25 us; the products' bytes
 // take 174 us.  8,000 products in runs of 8, 1,000 warps' work: 66 -> 42 us.
-// What is left is latency: the FP64 tensor pipe is 33-41 % busy and the issue
-// slots 30-40 %.  More warps an SM lose their cache lines to each other before
+// What is left is latency: the FP64 tensor pipe is 43 % busy and the issue
+// slots 28 %.  More warps an SM lose their cache lines to each other before
 // a line's second fragment is read (4 CTAs an SM, 32 x 32 blocks: 158 us
 // against 150 with 3).  Loads of 8 k at a time: 405 us; of 16 k, 422; of 16
 // or 20 k in the narrow shapes, 405 and 398.  A kernel for each shape let the
