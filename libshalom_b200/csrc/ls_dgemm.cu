@@ -247,8 +247,8 @@ __device__ __forceinline__ DsPart ds_part(bool along_k, bool wide, int lane, uin
 }
 template <int N>
 __device__ __forceinline__ void ds_load(double (&v)[N], const DsPart &d, const double *p, long sr,
-                                        long sk, int rows, int k0, int K) {
-  const char *q = reinterpret_cast<const char *>(p + d.r * sr + (k0 + d.k) * sk);
+                                        long sk, int rows, unsigned k0, unsigned K) {
+  const char *q = reinterpret_cast<const char *>(p + d.r * sr + (long)(k0 + d.k) * sk);
   const long step = 8 * (d.dr * sr + d.dk * sk);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(DS_WARPS * 32, DS_PER_SM)
   };
   fetch_next_entry();
   double v16[DS_KB / 2], v32[DS_KB];
-  int k0 = 0;
+  unsigned k0 = 0;  // (unsigned: K may be close to 2^31)
   auto load = [&]() {  // block k0 of product w
     auto get = [&](int k) { return __shfl_sync(FULL, w, k); };
     auto get64 = [&](int k) { return (uint64_t)get(k + 1) << 32 | get(k); };
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(DS_WARPS * 32, DS_PER_SM)
     const int M = (int)get(6), N = (int)get(7), transb = (int)get(9);
     const int K0 = max(0, (int)get(8)), lda = (int)get(10), ldb = (int)get(11);
     const long la = lda > 0 ? lda : K0, lb = ldb > 0 ? ldb : transb ? K0 : N;
-    const int K = M > 0 && N > 0 ? K0 : 0;
+    const unsigned K = M > 0 && N > 0 ? K0 : 0;
     const long br = transb ? lb : 1, bk = transb ? 1 : lb;
     if (N > 16) {
       const int m0 = u < two && (u & 1) ? 16 : 0;
@@ -344,7 +344,8 @@ __global__ void __launch_bounds__(DS_WARPS * 32, DS_PER_SM)
     // the block in the registers belongs to this product:
     auto get = [&](int k) { return __shfl_sync(FULL, w, k); };
     auto get64 = [&](int k) { return (uint64_t)get(k + 1) << 32 | get(k); };
-    const int M = (int)get(6), N = (int)get(7), K = max(0, (int)get(8)), transb = (int)get(9);
+    const int M = (int)get(6), N = (int)get(7), transb = (int)get(9);
+    const unsigned K = max(0, (int)get(8));
     const bool cols32 = N > 16;
     if (cols32) {
       ds_store(v16, ds_part(true, false, lane, a16));
@@ -372,7 +373,7 @@ __global__ void __launch_bounds__(DS_WARPS * 32, DS_PER_SM)
             c[i][j] = C[(m + i * tm) * ldc + n + j * tn];
         }
     }
-    const int kcnt = min(DS_KB, K - k0);
+    const int kcnt = (int)min((unsigned)DS_KB, K - k0);
     if (k0 == 0) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)

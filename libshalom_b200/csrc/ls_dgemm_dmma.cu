@@ -85,7 +85,7 @@ __device__ __forceinline__ void st_if(char *p, double v, bool on) {
 // never stored.
 template <bool TRANSB, int FM, int FN>
 __device__ __forceinline__ void dm_product(double (&acc)[FM][FN][2], const double *A,
-                                           const double *B, int M, int N, int K, long lda,
+                                           const double *B, int M, int N, unsigned K, long lda,
                                            long ldb, double alpha, int lane) {
   const int g = lane >> 2, q = lane & 3;
   const int MF = (M + 7) >> 3, NF = (N + 7) >> 3;
@@ -100,7 +100,7 @@ __device__ __forceinline__ void dm_product(double (&acc)[FM][FN][2], const doubl
 #pragma unroll
   for (int f = 0; f < FN; ++f) bc[f] = min(8 * f + g, N - 1);
 #pragma unroll 1
-  for (int k0 = 0; k0 < K; k0 += 4 * DM_KB) {
+  for (unsigned k0 = 0; k0 < K; k0 += 4 * DM_KB) {  // (unsigned: K may be close to 2^31)
     double a[DM_KB][FM], b[DM_KB][FN];
 #pragma unroll
     for (int f = 0; f < FM; ++f) {

@@ -17,7 +17,7 @@ using F128 = FlexCfg<64, 128>;
 
 // edge of tile t of `tiles` that cover `n` evenly, in steps of 4
 __host__ __device__ __forceinline__ int flex_edge(int n, int tiles) {
-  return ((n + tiles - 1) / tiles + 3) / 4 * 4;
+  return (int)(((long)n + tiles - 1) / tiles + 3) / 4 * 4;
 }
 
 // ---------------------------------------------------------------------------
@@ -77,8 +77,8 @@ struct FlexPlan {
 
 __device__ __forceinline__ bool fg_wide(int M, int N) { return M > 32 && N > 64; }
 __device__ __forceinline__ void fg_tiles(int M, int N, int *tiles_m, int *tiles_n) {
-  *tiles_m = (M + 63) / 64;
-  *tiles_n = fg_wide(M, N) ? (N + 127) / 128 : (N + 63) / 64;
+  *tiles_m = (int)((M + 63L) / 64);
+  *tiles_n = (int)(fg_wide(M, N) ? (N + 127L) / 128 : (N + 63L) / 64);
 }
 
 // items, class and length of the run starting at entry i (0 items: empty C)
