@@ -1199,24 +1199,28 @@ constexpr int GRP_CLASSES = 64;  // work classes (total K slabs of the run, capp
 // either: k_tc_grouped is faster on them (128 x 128 x 512 NT, 1,500 products:
 // 352 against 502 us; 256^3 NT, 1,000: 463 against 584 us), but as a second
 // kernel it only pays when there are enough of them to fill the machine.
-enum : int { GRP_SMALL = 0, GRP_LARGE = 1, GRP_EITHER = 2, GRP_EMPTY = 3 };
+// Small runs with a product of several K chunks that reads C have a list of their
+// own (HOLD).
+enum : int { GRP_SMALL = 0, GRP_HOLD = 1, GRP_LARGE = 2, GRP_LISTS = 3, GRP_EMPTY = 3 };
 constexpr int GRP_SMALL_EDGE = 256;
 constexpr int GRP_SMALL_TILES =
-    (GRP_SMALL_EDGE / SM_SMALL_TM) * (GRP_SMALL_EDGE / SM_SMALL_TN);
-constexpr long GRP_SMALL_MAX_COUNT = 1L << 24;  // 1 GB of items
-static_assert(GRP_SMALL_TILES <= 8, "an item word holds three bits of tile");
+    (GRP_SMALL_EDGE / SM_SUM_ROWS) * (GRP_SMALL_EDGE / SM_SMALL_TN);
+constexpr long GRP_SMALL_MAX_COUNT = 1L << 24;  // 2 GB of items
+static_assert(GRP_SMALL_TILES <= 16 && GRP_HOLD == 1, "an item word holds four bits of tile");
 
 // workspace layout of the plan (unsigned words)
 struct GrpPlan {
-  unsigned *class_n;     // [4][GRP_CLASSES] per class: items of the small runs, the large
-                         // runs, items of the runs that can be either, those runs
-  unsigned *class_off;   // [2][GRP_CLASSES] first sorted slot of each class (small, large)
-  unsigned *class_fill;  // [2][GRP_CLASSES] slots taken so far
-  unsigned *n_items;     // [2] items of the small-product kernel, runs of k_tc_grouped
+  unsigned *class_n;     // [6][GRP_CLASSES] per class: items of the small and of the hold
+                         // runs, the large runs; then, of the runs that can be either, the
+                         // same items and the runs
+  unsigned *class_off;   // [3][GRP_CLASSES] first sorted slot of each class (lists by kind)
+  unsigned *class_fill;  // [3][GRP_CLASSES] slots taken so far
+  unsigned *n_items;     // [3] items of the small-product kernel, runs of k_tc_grouped
   unsigned *counter;     // [1] work counter of the small-product kernel
   unsigned *either_large;  // [1] where the runs that can be either go
   unsigned either_min;     // runs that can be either for them to go to k_tc_grouped
-  uint2 *items;          // [GRP_SMALL_TILES * count]; null: every run is large
+  uint2 *items;          // [n_slots]: small upwards, hold downwards; null: every run is large
+  long n_slots;          // GRP_SMALL_TILES * count
   unsigned *run_first;   // [count] first entry of the large run in sorted slot s
   unsigned *run_len;     // [count]
 };
@@ -1237,30 +1241,35 @@ __device__ __forceinline__ bool grp_run_start(const LibShalom_sgemm_entry *e, lo
   return i == 0 || e[i].C != e[i - 1].C;
 }
 
-// The run starting at entry i: K work (capped class index), length, kernel
-// and tiles in the small-product kernel
+// The run starting at entry i: K work (capped class index), length, kernel,
+// tiles in the small-product kernel, and whether k_tc_grouped can take it too
 __device__ __forceinline__ int grp_run_class(const LibShalom_sgemm_entry *e, long count, long i,
-                                             bool with_small, long *len, int *kind, int *tiles) {
+                                             bool with_small, long *len, int *kind, int *tiles,
+                                             bool *either) {
   const int M = e[i].M, N = e[i].N;
   // share of the 128 x 128 tiles that C fills, at least 85 %
   const bool full = (long)M * N * 20 >= 17L * ((M + 127) / 128) * ((N + 127) / 128) * 16384;
-  bool fits = M <= GRP_SMALL_EDGE && N <= GRP_SMALL_EDGE, either = true;
+  bool fits = M <= GRP_SMALL_EDGE && N <= GRP_SMALL_EDGE, hold = false;
+  *either = true;
   long slabs = 0, j = i;
   do {
     const LibShalom_sgemm_entry &x = e[j];
+    hold = hold || (x.K > SM_SMALL_CHUNK && x.beta != 0.0f);
     slabs += max(1, (x.K + TC_BK - 1) / TC_BK);
     fits = fits && max(x.K, max(x.lda, x.ldb)) < (1 << 30);
     const int lda = x.lda > 0 ? x.lda : x.K, ldb = x.ldb > 0 ? x.ldb : x.transb ? x.K : N;
-    either = either && (((uintptr_t)x.A | (uintptr_t)x.B) & 15) == 0 && ((lda | ldb) & 3) == 0 &&
-             ((x.transb && x.K >= 128 && full) || (x.K > 256 && M >= 128));
+    *either = *either && (((uintptr_t)x.A | (uintptr_t)x.B) & 15) == 0 && ((lda | ldb) & 3) == 0 &&
+              ((x.transb && x.K >= 128 && full) || (x.K > 256 && M >= 128));
     ++j;
   } while (j < count && e[j].C == e[i].C);
   *len = j - i;
-  *tiles = ((M + SM_SMALL_TM - 1) / SM_SMALL_TM) * ((N + SM_SMALL_TN - 1) / SM_SMALL_TN);
-  *kind = M <= 0 || N <= 0                                ? GRP_EMPTY
-          : !with_small || !fits || j - i >= (1L << 28) ? GRP_LARGE
-          : either                                        ? GRP_EITHER
-                                                          : GRP_SMALL;
+  const int edge_m = hold ? SM_SUM_ROWS : SM_SMALL_TM;
+  *tiles = ((M + edge_m - 1) / edge_m) * ((N + SM_SMALL_TN - 1) / SM_SMALL_TN);
+  *kind = M <= 0 || N <= 0                              ? GRP_EMPTY
+          : !with_small || !fits || j - i >= (1L << 27) ? GRP_LARGE
+          : hold                                        ? GRP_HOLD
+                                                        : GRP_SMALL;
+  *either = *either && (*kind == GRP_SMALL || *kind == GRP_HOLD);
   return (int)min(slabs, (long)GRP_CLASSES - 1);
 }
 
@@ -1269,88 +1278,96 @@ __device__ __forceinline__ int grp_run_class(const LibShalom_sgemm_entry *e, lon
 // of the classes took 17 us on 50,000 products)
 __global__ void __launch_bounds__(256)
     k_grp_count(const LibShalom_sgemm_entry *e, long count, GrpPlan pl) {
-  static_assert(4 * GRP_CLASSES == 256, "one thread a class");
-  __shared__ unsigned n[4 * GRP_CLASSES];
+  constexpr int NC = 2 * GRP_LISTS * GRP_CLASSES;
+  __shared__ unsigned n[NC];
   chain_next();
-  n[threadIdx.x] = 0;
+  for (int c = threadIdx.x; c < NC; c += 256) n[c] = 0;
   __syncthreads();
   for (long i = blockIdx.x * 256L + threadIdx.x; i < count; i += gridDim.x * 256L) {
     if (!grp_run_start(e, i)) continue;
     long len;
     int kind, tiles;
-    const int cls = grp_run_class(e, count, i, pl.items != nullptr, &len, &kind, &tiles);
-    if (kind == GRP_SMALL) atomicAdd(&n[cls], (unsigned)tiles);
-    if (kind == GRP_LARGE) atomicAdd(&n[GRP_CLASSES + cls], 1u);
-    if (kind == GRP_EITHER) {
-      atomicAdd(&n[2 * GRP_CLASSES + cls], (unsigned)tiles);
-      atomicAdd(&n[3 * GRP_CLASSES + cls], 1u);
-    }
+    bool either;
+    const int cls = grp_run_class(e, count, i, pl.items != nullptr, &len, &kind, &tiles, &either);
+    if (kind == GRP_EMPTY) continue;
+    unsigned *at = n + cls + (either ? GRP_LISTS * GRP_CLASSES : 0);
+    atomicAdd(at + kind * GRP_CLASSES, kind == GRP_LARGE ? 1u : (unsigned)tiles);
+    if (either) atomicAdd(at + GRP_LARGE * GRP_CLASSES, 1u);
   }
   __syncthreads();
-  if (n[threadIdx.x]) atomicAdd(&pl.class_n[threadIdx.x], n[threadIdx.x]);
+  for (int c = threadIdx.x; c < NC; c += 256)
+    if (n[c]) atomicAdd(&pl.class_n[c], n[c]);
 }
 
-// pass 2: first sorted slot of every class, heaviest class first (one block of
-// GRP_CLASSES threads)
-__global__ void __launch_bounds__(GRP_CLASSES) k_grp_offsets(GrpPlan pl) {
-  __shared__ unsigned n[4][GRP_CLASSES];
-  __shared__ int s_large;
+// pass 2: first sorted slot of every class, heaviest class first (one block,
+// one thread a class of a list)
+constexpr int GRP_OFF_THREADS = GRP_LISTS * GRP_CLASSES;
+__global__ void __launch_bounds__(GRP_OFF_THREADS) k_grp_offsets(GrpPlan pl) {
+  static_assert(GRP_CLASSES == 64, "two warps a list");
+  __shared__ unsigned either_runs[2], sums[2 * GRP_LISTS];
   chain_wait();
   chain_next();
-  const int c = threadIdx.x;
-  for (int k = 0; k < 4; ++k) n[k][c] = pl.class_n[k * GRP_CLASSES + c];
-  __syncthreads();
-  if (c == 0) {
-    unsigned runs = 0;
-    for (int i = 0; i < GRP_CLASSES; ++i) runs += n[3][i];
-    s_large = runs >= pl.either_min;
-    *pl.either_large = s_large;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int l = tid / GRP_CLASSES, at = l * GRP_CLASSES + GRP_CLASSES - 1 - tid % GRP_CLASSES;
+  unsigned own = pl.class_n[at];
+  const unsigned either = pl.class_n[GRP_LISTS * GRP_CLASSES + at];
+  if (l == GRP_LARGE) {
+    const unsigned runs = __reduce_add_sync(0xffffffffu, either);
+    if (lane == 0) either_runs[warp & 1] = runs;
   }
   __syncthreads();
-  unsigned before[2] = {0, 0};
-  for (int i = GRP_CLASSES - 1; i >= c; --i) {
-    const unsigned s = n[0][i] + (s_large ? 0u : n[2][i]), l = n[1][i] + (s_large ? n[3][i] : 0u);
-    if (i > c) {
-      before[0] += s;
-      before[1] += l;
-    } else if (c == 0) {
-      pl.n_items[0] = before[0] + s;
-      pl.n_items[1] = before[1] + l;
-    }
+  const bool large = either_runs[0] + either_runs[1] >= pl.either_min;
+  if (tid == 0) *pl.either_large = large;
+  if ((l == GRP_LARGE) == large) own += either;
+  unsigned upto = own;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned v = __shfl_up_sync(0xffffffffu, upto, d);
+    if (lane >= d) upto += v;
   }
-  pl.class_off[c] = before[0];
-  pl.class_off[GRP_CLASSES + c] = before[1];
+  if (lane == 31) sums[warp] = upto;
+  __syncthreads();
+  if (warp & 1) upto += sums[warp - 1];
+  pl.class_off[at] = upto - own;
+  if ((warp & 1) && lane == 31) pl.n_items[l] = upto;
 }
 
 // pass 3: every item takes a slot in its class's range
 __global__ void __launch_bounds__(256)
     k_grp_place(const LibShalom_sgemm_entry *e, long count, GrpPlan pl) {
-  __shared__ unsigned n[2 * GRP_CLASSES], base[2 * GRP_CLASSES];
+  constexpr int NC = GRP_LISTS * GRP_CLASSES;
+  static_assert(NC <= 256, "one thread a class");
+  __shared__ unsigned n[NC], base[NC];
   chain_wait();
   chain_next();
   const bool either_large = *pl.either_large != 0;
   const int tid = threadIdx.x;
   for (long i0 = blockIdx.x * 256L; i0 < count; i0 += gridDim.x * 256L) {
-    if (tid < 2 * GRP_CLASSES) n[tid] = 0;
+    if (tid < NC) n[tid] = 0;
     __syncthreads();
     const long i = i0 + tid;
     long len = 0;
     int kind = GRP_EMPTY, tiles = 0, cls = 0;
-    if (i < count && grp_run_start(e, i))
-      cls = grp_run_class(e, count, i, pl.items != nullptr, &len, &kind, &tiles);
-    const bool large = kind == GRP_LARGE || (kind == GRP_EITHER && either_large);
-    if (large) cls += GRP_CLASSES;
-    const unsigned rank = kind == GRP_EMPTY ? 0 : atomicAdd(&n[cls], large ? 1u : (unsigned)tiles);
+    bool either;
+    if (i < count && grp_run_start(e, i)) {
+      cls = grp_run_class(e, count, i, pl.items != nullptr, &len, &kind, &tiles, &either);
+      if (either && either_large) kind = GRP_LARGE;
+      cls += kind * GRP_CLASSES;
+    }
+    const unsigned rank =
+        kind == GRP_EMPTY ? 0 : atomicAdd(&n[cls], kind == GRP_LARGE ? 1u : (unsigned)tiles);
     __syncthreads();
-    if (tid < 2 * GRP_CLASSES && n[tid])
-      base[tid] = pl.class_off[tid] + atomicAdd(&pl.class_fill[tid], n[tid]);
+    if (tid < NC && n[tid]) base[tid] = pl.class_off[tid] + atomicAdd(&pl.class_fill[tid], n[tid]);
     __syncthreads();
-    if (large) {
+    if (kind == GRP_LARGE) {
       pl.run_first[base[cls] + rank] = (unsigned)i;
       pl.run_len[base[cls] + rank] = (unsigned)len;
     } else if (kind != GRP_EMPTY) {
-      for (int t = 0; t < tiles; ++t)
-        pl.items[base[cls] + rank + t] = make_uint2((unsigned)i, (unsigned)len << 3 | (unsigned)t);
+      for (int t = 0; t < tiles; ++t) {
+        const long at = (long)base[cls] + rank + t;
+        pl.items[kind == GRP_HOLD ? pl.n_slots - 1 - at : at] =
+            make_uint2((unsigned)i, (unsigned)len << 5 | (unsigned)kind << 4 | (unsigned)t);
+      }
     }
     __syncthreads();
   }
@@ -2018,10 +2035,11 @@ int tc_launch(TcProblem &p, int mode) {
     sa.M = p.M; sa.N = p.N; sa.K = p.K; sa.transb = p.transb;
     sa.alpha = p.alpha; sa.beta = p.beta;
     sa.tiles_n = (int)cdiv(p.N, SM_SMALL_TN);
-    sa.tiles = (int)cdiv(p.M, SM_SMALL_TM) * sa.tiles_n;
+    const bool hold = p.K > SM_SMALL_CHUNK && p.beta != 0.0f;
+    sa.tiles = (int)cdiv(p.M, hold ? SM_SUM_ROWS : SM_SMALL_TM) * sa.tiles_n;
     sa.n_items = (long)sa.tiles * p.count;
     sa.err = p.err;
-    const int rc = tc_small_launch(sa, true, mode);
+    const int rc = tc_small_launch(sa, true, hold, mode);
     if (rc) return rc;
   } else if (tma) {
     const bool wide = !drain && wa.c_tma;
@@ -2206,20 +2224,21 @@ int tc_sgemm_grouped(const LibShalom_sgemm_entry *entries, long count, int mode)
   unsigned *w = static_cast<unsigned *>(ws);
   GrpPlan pl;
   pl.class_n = w;
-  pl.class_off = w + 4 * GRP_CLASSES;
-  pl.class_fill = w + 6 * GRP_CLASSES;
-  pl.n_items = w + 8 * GRP_CLASSES;
-  pl.counter = pl.n_items + 2;
-  pl.either_large = pl.n_items + 3;
+  pl.class_off = pl.class_n + 2 * GRP_LISTS * GRP_CLASSES;
+  pl.class_fill = pl.class_off + GRP_LISTS * GRP_CLASSES;
+  pl.n_items = pl.class_fill + GRP_LISTS * GRP_CLASSES;
+  pl.counter = pl.n_items + GRP_LISTS;
+  pl.either_large = pl.counter + 1;
   pl.either_min = 2u * (unsigned)st.num_sms;
   pl.items = with_small ? reinterpret_cast<uint2 *>(w + GRP_HEADER) : nullptr;
+  pl.n_slots = (long)GRP_SMALL_TILES * count;
   pl.run_first = w + GRP_HEADER + (with_small ? item_words : 0);
   pl.run_len = pl.run_first + count;
   LS_CUDA_TRY(cudaMemsetAsync(w, 0, GRP_HEADER * sizeof(unsigned), st.stream));
   const int pgrid = (int)std::max(1L, std::min(cdiv(count, 256), (long)st.num_sms * 8));
   k_grp_count<<<pgrid, 256, 0, st.stream>>>(entries, count, pl);
   LS_CUDA_TRY(cudaGetLastError());
-  int rc = launch_chained(k_grp_offsets, 1, GRP_CLASSES, 0, st.stream, pl);
+  int rc = launch_chained(k_grp_offsets, 1, GRP_OFF_THREADS, 0, st.stream, pl);
   if (!rc) rc = launch_chained(k_grp_place, pgrid, 256, 0, st.stream, entries, count, pl);
   if (rc) return rc;
 
@@ -2229,10 +2248,11 @@ int tc_sgemm_grouped(const LibShalom_sgemm_entry *entries, long count, int mode)
     TcSmallArgs sa{};
     sa.entries = entries;
     sa.items = pl.items;
+    sa.n_slots = pl.n_slots;
     sa.n_items_dev = pl.n_items;
     sa.counter = pl.counter;
     sa.err = reinterpret_cast<unsigned *>(errp);
-    rc = tc_small_launch(sa, false, mode);
+    rc = tc_small_launch(sa, false, false, mode);
     if (rc) return rc;
   }
   GrpArgs g;
@@ -2240,7 +2260,7 @@ int tc_sgemm_grouped(const LibShalom_sgemm_entry *entries, long count, int mode)
   g.count = count;
   g.run_first = pl.run_first;
   g.run_len = pl.run_len;
-  g.n_runs = pl.n_items + 1;
+  g.n_runs = pl.n_items + GRP_LARGE;
   g.err = reinterpret_cast<unsigned *>(errp);
   g.kc_slabs = 128 / TC_BK;
   auto kern = mode == LIBSHALOM_PREC_BF16X6 ? k_tc_grouped<3> : k_tc_grouped<2>;

@@ -20,13 +20,19 @@ int tc_sgemm_grouped(const LibShalom_sgemm_entry *entries, long count, int mode)
 
 // Tiles of the small-product kernel (ls_tc_small.cu): C rows and columns.
 constexpr int SM_SMALL_TM = 64, SM_SMALL_TN = 128;
+// Its K chunks, and the rows of a tile whose chunk sums fit beside the
+// accumulators (tiles of its HOLD loop, for products of several chunks that
+// read C).
+constexpr int SM_SMALL_CHUNK = 128, SM_SUM_ROWS = 32;
 
 // Work of the small-product kernel.  Grouped: items {first entry of the run,
-// products << 3 | tile} in device memory.  Uniform: GEMM g of the batch at
-// A + g * sA etc., `tiles` tiles each.
+// products << 5 | hold << 4 | tile} in device memory, n_items_dev[0] upwards from
+// items[0] and, of the HOLD loop, n_items_dev[1] downwards from items[n_slots - 1].
+// Uniform: GEMM g of the batch at A + g * sA etc., `tiles` tiles each.
 struct TcSmallArgs {
   const LibShalom_sgemm_entry *entries;
   const uint2 *items;
+  long n_slots;
   const unsigned *n_items_dev;
   unsigned *counter;  // zeroed before the launch
   const float *A, *B;
@@ -36,7 +42,8 @@ struct TcSmallArgs {
   float alpha, beta;
   unsigned *err;  // device status word (bounded waits)
 };
-int tc_small_launch(const TcSmallArgs &a, bool uniform, int mode);
+// hold: of a uniform batch
+int tc_small_launch(const TcSmallArgs &a, bool uniform, bool hold, int mode);
 
 // Runs the bounded-wait self-check kernel (an mbarrier nothing arrives at);
 // returns LIBSHALOM_ERR_DEVICE_TIMEOUT when its waits expired and reported.
