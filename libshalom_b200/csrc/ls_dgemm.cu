@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(DS_WARPS * 32, DS_PER_SM)
   load();
 
   double c[4][4], acc[4][4];
+  long ldc = 0;  // of the run: its first product's
   bool new_run = true;
 #pragma unroll 1
   for (;;) {
@@ -361,9 +362,9 @@ __global__ void __launch_bounds__(DS_WARPS * 32, DS_PER_SM)
     const double alpha = __longlong_as_double((long long)get64(14));
     const double beta = __longlong_as_double((long long)get64(16));
     double *const C = reinterpret_cast<double *>(get64(4));
-    const int ldc0 = (int)get(12);
-    const long ldc = ldc0 > 0 ? ldc0 : N;
     if (new_run) {
+      const int ldc0 = (int)get(12);
+      ldc = ldc0 > 0 ? ldc0 : N;
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
