@@ -175,7 +175,10 @@ LIBSHALOM_API int LibShalom_set_tma(int enable);
  * LIBSHALOM_SUCCESS would mean the expiry went unreported. */
 LIBSHALOM_API int LibShalom_selftest_wait_expiry(int iterations);
 
-/* Release the library's device workspace and cached plans. */
+/* Release the library's device workspace and cached plans.  (The workspace
+ * grows with the largest call so far.  Calls may be captured into a caller's CUDA
+ * graph in asynchronous mode, growth included; a workspace that such a graph
+ * names is kept until this call, after which the graph must not be launched.) */
 LIBSHALOM_API void LibShalom_finalize(void);
 
 /* ---------------------------------------------------------------------- */

@@ -56,26 +56,54 @@ int ensure_device() {
   return LIBSHALOM_SUCCESS;
 }
 
+// Whether the caller is capturing the library's stream into a graph (the null
+// stream cannot be captured; the graph cache's own captures set own_capture).
+static bool caller_captures() {
+  State &st = state();
+  if (!st.stream || st.stream == cudaStreamLegacy || st.own_capture) return false;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st.stream, &status) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return status == cudaStreamCaptureStatusActive;
+}
+
+// A buffer that a caller's graph names is kept until finalize when it is
+// outgrown (each at most half as large as the next: together less than the one
+// in use); one that no graph names is freed once the stream is done with it.
 int workspace(size_t bytes, void **out) {
   State &st = state();
   if (bytes < 256) bytes = 256;
+  const bool captured = caller_captures();
   if (st.ws && st.ws_bytes >= bytes && st.ws_device == st.device) {
+    st.ws_in_graph = st.ws_in_graph || captured;
     *out = st.ws;
     return LIBSHALOM_SUCCESS;
   }
-  if (st.ws) {
+  size_t want = std::max(bytes, (size_t)1 << 20);
+  if (st.ws && (st.ws_in_graph || captured || st.own_capture)) {
+    // (the stream cannot be waited for while it is captured)
+    want = std::max(want, 2 * st.ws_bytes);
+    st.ws_kept.push_back(st.ws);
+  } else if (st.ws) {
     // kernels queued earlier may still read the old buffer
     LS_CUDA_TRY(cudaStreamSynchronize(st.stream));
     cudaFree(st.ws);
-    st.ws = nullptr;
-    st.ws_bytes = 0;
   }
-  size_t want = std::max(bytes, (size_t)1 << 20);
-  if (cudaMalloc(&st.ws, want) != cudaSuccess) {
+  st.ws = nullptr;
+  st.ws_bytes = 0;
+  // cudaMalloc is no stream operation: the relaxed mode allows it in a capture
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  LS_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+  const cudaError_t e = cudaMalloc(&st.ws, want);
+  LS_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+  if (e != cudaSuccess) {
     cudaGetLastError();
     st.ws = nullptr;
     return LIBSHALOM_ERR_ALLOC;
   }
+  st.ws_in_graph = captured;
   st.ws_bytes = want;
   st.ws_device = st.device;
   ++st.ws_generation;  // graphs captured with the old buffer are stale
@@ -293,7 +321,9 @@ static int gemm_cached(int kind, int transa, int transb, T *C, const T *A, const
   const int sync = st.sync;
   st.sync = 0;  // no host synchronisation inside the capture
   LS_CUDA_TRY(cudaStreamBeginCapture(st.stream, cudaStreamCaptureModeThreadLocal));
+  st.own_capture = true;
   rc = gemm_common<T>(transa, transb, C, A, B, M, N, K, mp);
+  st.own_capture = false;
   cudaGraph_t graph = nullptr;
   const cudaError_t ce = cudaStreamEndCapture(st.stream, &graph);
   st.sync = sync;
@@ -921,7 +951,7 @@ void LibShalom_finalize(void) {
   State &st = state();
   // calls still pending in a deferred section run before anything is freed
   const int flushed = flush_deferred();
-  if (st.ws || st.fe) cudaStreamSynchronize(st.stream);
+  if (st.ws || st.fe || !st.ws_kept.empty()) cudaStreamSynchronize(st.stream);
   graph_cache_clear();
   if (st.ring_busy && st.ring_ev) cudaEventSynchronize(st.ring_ev);
   if (st.ring_ev) cudaEventDestroy(st.ring_ev);
@@ -942,6 +972,9 @@ void LibShalom_finalize(void) {
     if (cur >= 0) cudaSetDevice(cur);
   }
   if (st.ws) cudaFree(st.ws);
+  for (void *p : st.ws_kept) cudaFree(p);
+  st.ws_kept.clear();
+  st.ws_in_graph = false;
   if (st.fe) cudaFree(st.fe);
   st.ws = nullptr;
   st.ws_bytes = 0;

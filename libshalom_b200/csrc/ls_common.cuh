@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include <mutex>
+#include <vector>
 
 #include "../../include/LibShalom.h"
 
@@ -57,6 +58,9 @@ struct State {
   void *ws = nullptr;
   size_t ws_bytes = 0;
   int ws_device = -1;
+  bool ws_in_graph = false;     // a caller's graph names the workspace
+  std::vector<void *> ws_kept;  // outgrown workspaces that callers' graphs name
+  bool own_capture = false;     // the graph cache is capturing
   // front-end buffer (stack entries, im2col columns): separate from the
   // workspace, which the GEMM paths the front ends call use themselves
   void *fe = nullptr;
@@ -90,9 +94,10 @@ State &state();
 // LIBSHALOM_* status.
 int ensure_device();
 
-// Device workspace of at least `bytes` bytes (grown on demand, stream
-// ordered: the caller's stream is synchronised before a regrow;
-// LibShalom_set_stream finishes the old stream's work before a switch).
+// Device workspace of at least `bytes` bytes (grown on demand, also while the
+// stream is captured; stream ordered: the caller's stream is synchronised before
+// a buffer is freed; LibShalom_set_stream finishes the old stream's work before a
+// switch).
 int workspace(size_t bytes, void **out);
 
 // Launches the drop-in calls recorded since LibShalom_defer_begin (on the
