@@ -1185,8 +1185,9 @@ int LibShalom_sconv2d_nchw(const float *x, long n, long c, long h, long w, const
   if (n < 0 || c <= 0 || h <= 0 || w <= 0 || oc <= 0 || kh <= 0 || kw <= 0 || sh <= 0 ||
       sw <= 0 || ph < 0 || pw < 0 || !x || !wt || !y)
     rc = LIBSHALOM_ERR_INVALID_VALUE;
-  const long oh = (h + 2 * ph - kh) / sh + 1, ow = (w + 2 * pw - kw) / sw + 1;
   if (!rc && (h + 2 * ph < kh || w + 2 * pw < kw)) rc = LIBSHALOM_ERR_INVALID_VALUE;
+  // (after the checks: a stride of 0 divides)
+  const long oh = rc ? 0 : (h + 2 * ph - kh) / sh + 1, ow = rc ? 0 : (w + 2 * pw - kw) / sw + 1;
   // the implicit GEMM indexes k = (ci, r, q) and p = (oy, ox) in int32
   const bool small_idx = c * kh * kw < INT32_MAX && oh * ow < INT32_MAX && c * h * w < INT32_MAX;
   if (!rc && n > 0 && state().precision == LIBSHALOM_PREC_FP32 && small_idx &&
