@@ -121,7 +121,9 @@ int finish_launch(const char *what);
 inline long cdiv(long a, long b) { return (a + b - 1) / b; }
 
 // Launch of a kernel that waits for its predecessor on the device
-// (chain_wait): its blocks are put in place while the predecessor runs.
+// (chain_wait): its blocks are put in place while the predecessor runs, except
+// under LibShalom_set_thread_nums, whose cap on resident CTAs two kernels at a
+// time would exceed.
 template <class... P, class... A>
 int launch_chained(void (*kern)(P...), long grid, int threads, size_t smem, cudaStream_t stream,
                    A... args) {
@@ -134,15 +136,17 @@ int launch_chained(void (*kern)(P...), long grid, int threads, size_t smem, cuda
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = &early;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = state().thread_cap > 0 ? 0 : 1;
   LS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
   return LIBSHALOM_SUCCESS;
 }
 
 #ifdef __CUDACC__
-// First statement of every thread of a kernel launched with launch_chained:
-// the kernels before it have completed and their writes are visible, so that
-// nothing it does, or a kernel after it, can overtake them.
+// The kernels before a kernel launched with launch_chained have completed and
+// their writes are visible.  Its threads call this first, so that nothing they
+// do, or a kernel after theirs, can overtake those kernels.  (k_flex_grouped for
+// the small list calls it last and says why: nothing it reads is written by the
+// one kernel that may still run, and the end of the call is what has to wait.)
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Lets the next kernel's blocks take the places that are left (after this
 // kernel's own blocks have all been placed).
