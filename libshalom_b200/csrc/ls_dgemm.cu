@@ -43,6 +43,7 @@
 #include "ls_common.cuh"
 #include "ls_dgemm_runs.cuh"
 #include "ls_simt_launch.h"
+#include "ls_sizes.h"
 
 namespace ls {
 
@@ -474,9 +475,9 @@ __global__ void __launch_bounds__(DR_THREADS, 6)
   const long n_runs = (long)*n_runs_p;
 
   auto tiles_of = [&](const LibShalom_dgemm_entry &e) {
-    return ((e.M + DR_T - 1) / DR_T) * ((e.N + DR_T - 1) / DR_T);
+    return ceil_div(e.M, DR_T) * ceil_div(e.N, DR_T);
   };
-  auto slabs_of = [&](const LibShalom_dgemm_entry &e) { return max(1, (max(0, e.K) + DR_T - 1) / DR_T); };
+  auto slabs_of = [&](const LibShalom_dgemm_entry &e) { return slabs(e.K, DR_T); };
 
   // advance a cursor to the next slab; returns false past the CTA's last run
   auto advance = [&](DCursor &c) -> bool {
@@ -504,7 +505,7 @@ __global__ void __launch_bounds__(DR_THREADS, 6)
     const unsigned f = run_first[c.r];
     const LibShalom_dgemm_entry &e0 = entries[f];
     const DJob jb = djob(entries[f + c.p]);
-    const int tiles_n = (e0.N + DR_T - 1) / DR_T;
+    const int tiles_n = ceil_div(e0.N, DR_T);
     const int m0 = (c.t / tiles_n) * DR_T, n0 = (c.t % tiles_n) * DR_T, k0 = c.k * DR_T;
     double *As = stage[b];
     double *Bs = stage[b] + DR_T * DR_P;
@@ -543,7 +544,7 @@ __global__ void __launch_bounds__(DR_THREADS, 6)
     const unsigned f = run_first[cur.r];
     const LibShalom_dgemm_entry &e0 = entries[f];
     const DJob jb = djob(entries[f + cur.p]);
-    const int tiles_n = (e0.N + DR_T - 1) / DR_T;
+    const int tiles_n = ceil_div(e0.N, DR_T);
     const int m0 = (cur.t / tiles_n) * DR_T, n0 = (cur.t % tiles_n) * DR_T;
     double *Crow0 = entries[f].C + (long)(m0 + 4 * ty) * (e0.ldc > 0 ? e0.ldc : e0.N) + n0 + 4 * tx;
     const int ldc = e0.ldc > 0 ? e0.ldc : e0.N;
@@ -583,7 +584,7 @@ __global__ void __launch_bounds__(DR_THREADS, 6)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = __fma_rn(av[i], bv[j], acc[i][j]);
     }
-    const bool product_done = cur.k + 1 >= max(1, (jb.K + DR_T - 1) / DR_T);
+    const bool product_done = cur.k + 1 >= slabs(jb.K, DR_T);
     if (product_done) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)

@@ -37,6 +37,7 @@
 
 #include "ls_f32x2.cuh"
 #include "ls_simt.cuh"
+#include "ls_sizes.h"
 
 namespace ls {
 
@@ -148,7 +149,7 @@ __device__ __forceinline__ void flex_tile(const FlexJob &j, int m0, int n0, int 
 #pragma unroll
     for (int q = 0; q < TN / 2; ++q) acc[i][q] = 0;
 
-  const int nslab = (int)(((unsigned)j.K + FX_KS - 1) / FX_KS);
+  const int nslab = ceil_div(j.K, FX_KS);
   if (nslab > 0) issue(0);
   simt_commit();
   for (int s = 0; s < nslab; ++s) {

@@ -7,6 +7,7 @@
 #include "ls_common.cuh"
 #include "ls_flex.cuh"
 #include "ls_simt_launch.h"
+#include "ls_sizes.h"
 
 namespace ls {
 
@@ -77,8 +78,8 @@ struct FlexPlan {
 
 __device__ __forceinline__ bool fg_wide(int M, int N) { return M > 32 && N > 64; }
 __device__ __forceinline__ void fg_tiles(int M, int N, int *tiles_m, int *tiles_n) {
-  *tiles_m = (int)((M + 63L) / 64);
-  *tiles_n = (int)(fg_wide(M, N) ? (N + 127L) / 128 : (N + 63L) / 64);
+  *tiles_m = ceil_div(M, 64);
+  *tiles_n = ceil_div(N, fg_wide(M, N) ? 128 : 64);
 }
 
 // items, class and length of the run starting at entry i (0 items: empty C)

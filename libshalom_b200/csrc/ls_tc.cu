@@ -33,6 +33,7 @@
 #include "ls_common.cuh"
 #include "ls_tc_launch.h"
 #include "ls_simt_launch.h"
+#include "ls_sizes.h"
 #include "ls_tc_ptx.cuh"
 
 namespace ls {
@@ -1235,7 +1236,7 @@ struct GrpArgs {
 };
 
 
-__device__ __forceinline__ int grp_tile_n(int N) { return min(TC_MAX_N, (N + 15) / 16 * 16); }
+__device__ __forceinline__ int grp_tile_n(int N) { return ceil_div(min(TC_MAX_N, N), 16) * 16; }
 
 __device__ __forceinline__ bool grp_run_start(const LibShalom_sgemm_entry *e, long i) {
   return i == 0 || e[i].C != e[i - 1].C;
@@ -1248,14 +1249,14 @@ __device__ __forceinline__ int grp_run_class(const LibShalom_sgemm_entry *e, lon
                                              bool *either) {
   const int M = e[i].M, N = e[i].N;
   // share of the 128 x 128 tiles that C fills, at least 85 %
-  const bool full = (long)M * N * 20 >= 17L * ((M + 127) / 128) * ((N + 127) / 128) * 16384;
+  const bool full = (long)M * N * 20 >= 17L * ceil_div(M, 128) * ceil_div(N, 128) * 16384;
   bool fits = M <= GRP_SMALL_EDGE && N <= GRP_SMALL_EDGE, hold = false;
   *either = true;
-  long slabs = 0, j = i;
+  long k_slabs = 0, j = i;
   do {
     const LibShalom_sgemm_entry &x = e[j];
     hold = hold || (x.K > SM_SMALL_CHUNK && x.beta != 0.0f);
-    slabs += max(1, (x.K + TC_BK - 1) / TC_BK);
+    k_slabs += slabs(x.K, TC_BK);
     fits = fits && max(x.K, max(x.lda, x.ldb)) < (1 << 30);
     const int lda = x.lda > 0 ? x.lda : x.K, ldb = x.ldb > 0 ? x.ldb : x.transb ? x.K : N;
     *either = *either && (((uintptr_t)x.A | (uintptr_t)x.B) & 15) == 0 && ((lda | ldb) & 3) == 0 &&
@@ -1264,13 +1265,13 @@ __device__ __forceinline__ int grp_run_class(const LibShalom_sgemm_entry *e, lon
   } while (j < count && e[j].C == e[i].C);
   *len = j - i;
   const int edge_m = hold ? SM_SUM_ROWS : SM_SMALL_TM;
-  *tiles = ((M + edge_m - 1) / edge_m) * ((N + SM_SMALL_TN - 1) / SM_SMALL_TN);
+  *tiles = ceil_div(M, edge_m) * ceil_div(N, SM_SMALL_TN);
   *kind = M <= 0 || N <= 0                              ? GRP_EMPTY
           : !with_small || !fits || j - i >= (1L << 27) ? GRP_LARGE
           : hold                                        ? GRP_HOLD
                                                         : GRP_SMALL;
   *either = *either && (*kind == GRP_SMALL || *kind == GRP_HOLD);
-  return (int)min(slabs, (long)GRP_CLASSES - 1);
+  return (int)min(k_slabs, (long)GRP_CLASSES - 1);
 }
 
 // pass 1: items per work class
@@ -1436,7 +1437,7 @@ __device__ __forceinline__ bool q_get(const unsigned char *smem, long j, GItem &
   it.ldc = s.ldc; it.m0 = s.m0; it.n0 = s.n0;
   it.alpha = s.alpha; it.beta = s.beta;
   it.tn = grp_tile_n(max(1, it.N));
-  it.nk = max(1, (it.K + TC_BK - 1) / TC_BK);
+  it.nk = slabs(it.K, TC_BK);
   return true;
 }
 
@@ -1539,8 +1540,8 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_tc_grouped(const GrpArgs g) {
         const int M = g.entries[first].M, N = g.entries[first].N;
         if (M > 0 && N > 0) {
           tn = grp_tile_n(N);
-          tiles_n = (N + tn - 1) / tn;
-          items = (long)((M + TC_BM - 1) / TC_BM) * tiles_n * len;
+          tiles_n = ceil_div(N, tn);
+          items = (long)ceil_div(M, TC_BM) * tiles_n * len;
         }
       }
       long incl = items;  // inclusive prefix of items over the lanes
