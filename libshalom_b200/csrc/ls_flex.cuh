@@ -5,7 +5,8 @@
 // threads of TM x TN outputs, laid out for the tile at hand, so a 52 x 104
 // half of a 104^3 product keeps 7 x 13 of 128 threads busy instead of a
 // quarter of a 128 x 128 tile's.  Several CTAs share an SM and hide each
-// other's latencies; a tile's K slabs go through a ring of two stages.
+// other's latencies; a tile's K slabs go through a ring of two stages (three on
+// 32 x 32 tiles, which are for batches too small to fill the SMs).
 //
 // Both operands are staged k-major ([k][m], [k][n]) by cp.async straight from
 // row-major global memory, whatever its layout: operands whose k runs along
@@ -23,7 +24,7 @@
 //
 // Bound by the shared-memory pipe (64^3: 74 % busy): the transposing
 // four-byte copies take some ten wavefronts each.  Tried instead, on 104^3 NT
-// (944 us) / the mixed batch in one list (1.55 ms): rows kept as they lie and read along
+// (944 us then) / the mixed batch in one list (1.55 ms then): rows kept as they lie and read along
 // k (967 us / 2.86 ms: a register move per pair of columns, more code),
 // transposition through registers without (1,533 us / 2.49 ms) and with a
 // slab of prefetch (1,341 us / 3.96 ms: spills), two loading warps a CTA
@@ -44,14 +45,19 @@ namespace ls {
 constexpr int FX_THREADS = 128;
 constexpr int FX_KS = 32;  // k per slab
 
-template <int MAXM_, int MAXN_>
+template <int MAXM_, int MAXN_, int STAGES_ = 2>
 struct FlexCfg {
-  static constexpr int MAXM = MAXM_, MAXN = MAXN_;
+  static constexpr int MAXM = MAXM_, MAXN = MAXN_, STAGES = STAGES_;
   static constexpr int PA = MAXM + 4, PB = MAXN + 4;  // pitches: 4 mod 32 words
   static constexpr int STAGE = FX_KS * (PA + PB);     // floats
-  static constexpr int SMEM = 2 * STAGE * 4;
+  static constexpr int SMEM = STAGES * STAGE * 4;
+  // ring position of slab s
+  static __device__ __forceinline__ int slot(int s) {
+    if constexpr (STAGES == 2) return s & 1;
+    else return s % STAGES;
+  }
   static_assert(PA % 32 == 4 && PB % 32 == 4, "transposing copies without bank conflicts");
-  static_assert(MAXM * PB <= 2 * STAGE, "the C tile goes through the ring");
+  static_assert(MAXM * PB <= STAGES * STAGE, "the C tile goes through the ring");
 };
 
 struct FlexJob {
@@ -119,6 +125,17 @@ __device__ __forceinline__ void fx_lds4(uint32_t a, float *v) {
                : "memory");
 }
 
+__device__ __forceinline__ float fx_ld(const float *p, bool on) {
+  float v;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+      "@p ld.global.f32 %0, [%1];\n\t}"
+      : "=f"(v)
+      : "l"(p), "r"((int)on)
+      : "memory");
+  return v;
+}
+
 // One product on one tile: C[m0.., n0..] = alpha A op(B) + beta C
 template <class Cfg, int TM, int TN>
 __device__ __forceinline__ void flex_tile(const FlexJob &j, int m0, int n0, int mrows, int ncols,
@@ -133,9 +150,10 @@ __device__ __forceinline__ void flex_tile(const FlexJob &j, int m0, int n0, int 
   const float *B = j.transb ? j.B + (long)n0 * j.ldb : j.B + n0;
   const bool vec_b = (reinterpret_cast<uintptr_t>(B) & 15) == 0 && (j.ldb & 3) == 0;
 
+  constexpr int AHEAD = Cfg::STAGES - 1;  // slabs on their way while one is multiplied
   auto issue = [&](int s) {
     const int k0 = s * FX_KS, kcnt = min(FX_KS, j.K - k0);
-    const uint32_t sa = sbase + (s & 1) * Cfg::STAGE * 4, sb = sa + FX_KS * PA * 4;
+    const uint32_t sa = sbase + Cfg::slot(s) * Cfg::STAGE * 4, sb = sa + FX_KS * PA * 4;
     fx_stage_k<PA>(sa, A + k0, j.lda, mrows, kcnt, warp, lane);
     if (j.transb) fx_stage_k<PB>(sb, B + k0, j.ldb, ncols, kcnt, warp, lane);
     else fx_stage_n<PB, Cfg::MAXN>(sb, B + (long)k0 * j.ldb, j.ldb, ncols, kcnt, vec_b, tid);
@@ -150,16 +168,19 @@ __device__ __forceinline__ void flex_tile(const FlexJob &j, int m0, int n0, int 
     for (int q = 0; q < TN / 2; ++q) acc[i][q] = 0;
 
   const int nslab = ceil_div(j.K, FX_KS);
-  if (nslab > 0) issue(0);
-  simt_commit();
-  for (int s = 0; s < nslab; ++s) {
-    if (s + 1 < nslab) issue(s + 1);
+#pragma unroll
+  for (int s = 0; s < AHEAD; ++s) {
+    if (s < nslab) issue(s);
     simt_commit();
-    simt_wait<1>();
+  }
+  for (int s = 0; s < nslab; ++s) {
+    if (s + AHEAD < nslab) issue(s + AHEAD);
+    simt_commit();
+    simt_wait<AHEAD>();
     __syncthreads();
     if (on) {
-      uint32_t pa = sbase + (s & 1) * Cfg::STAGE * 4 + ty * 16;
-      uint32_t pb = sbase + ((s & 1) * Cfg::STAGE + FX_KS * PA) * 4 + tx * 16;
+      uint32_t pa = sbase + Cfg::slot(s) * Cfg::STAGE * 4 + ty * 16;
+      uint32_t pb = sbase + (Cfg::slot(s) * Cfg::STAGE + FX_KS * PA) * 4 + tx * 16;
       const int kcnt = min(FX_KS, j.K - s * FX_KS);
       auto step = [&](uint32_t qa, uint32_t qb) {
         float a[TM], b[TN];
@@ -206,13 +227,32 @@ __device__ __forceinline__ void flex_tile(const FlexJob &j, int m0, int n0, int 
     }
   }
   __syncthreads();
-  for (int r = warp; r < mrows; r += FX_THREADS / 32) {
-    float *crow = j.C + (long)(m0 + r) * j.ldc + n0;
-    for (int c = lane; c < ncols; c += 32) {
-      float v = smem[r * PB + c];
-      if (j.beta != 0.0f) v = __fmaf_rn(j.beta, crow[c], v);
-      crow[c] = v;
+  // eight elements a thread at a time, C read for all of them first: one by one,
+  // the loads of a 64 x 64 tile were a chain of 32 (a run of 128 products of 64^3
+  // 1,454 us instead of 914, 10,000 products of 24^3 49 instead of 39)
+  constexpr int W = FX_THREADS / 32, Q = Cfg::MAXN / 32, U = 8 / Q;
+  const bool read = j.beta != 0.0f;
+  for (int r0 = warp; r0 < mrows; r0 += W * U) {
+    float *c0 = j.C + (long)(m0 + r0) * j.ldc + n0 + lane;
+    float cv[U][Q];
+    if (read) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+          cv[u][q] = fx_ld(c0 + (long)(u * W) * j.ldc + q * 32,
+                           r0 + u * W < mrows && lane + q * 32 < ncols);
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        if (r0 + u * W < mrows && lane + q * 32 < ncols) {
+          float v = smem[(r0 + u * W) * PB + lane + q * 32];
+          if (read) v = __fmaf_rn(j.beta, cv[u][q], v);
+          c0[(long)(u * W) * j.ldc + q * 32] = v;
+        }
+      }
   }
   __syncthreads();  // the ring is free for the next tile
 }

@@ -13,6 +13,7 @@ namespace ls {
 
 namespace {
 
+using F32 = FlexCfg<32, 32, 3>;
 using F64 = FlexCfg<64, 64>;
 using F128 = FlexCfg<64, 128>;
 
@@ -32,6 +33,10 @@ struct FlexUniform {
   float alpha, beta;
   int tiles, tiles_n, edge_m, edge_n;
 };
+
+// 32 x 32 tiles an SM (as many as it holds) up to which a batch takes them: 64^3
+// alone 8.2 -> 5.4 us, 128^3 14.3 -> 8.2, 222 products of 64^3 11.1 -> 9.2
+constexpr long FU_FEW = 6;
 
 template <class Cfg, int TM, int TN, int PER_SM>
 __global__ void __launch_bounds__(FX_THREADS, PER_SM) k_flex_uniform(const FlexUniform u) {
@@ -56,18 +61,18 @@ constexpr int FG_CLASSES = 64;  // work classes: half octaves of M N K a part
 constexpr int FG_PARTS = 16;    // a run's tiles are dealt to at most 16 items
 // Wide items a CTA up to which the small list's blocks start beside the wide
 // list's: their tails fill each other, but the two share an SM's L1 from then
-// on.  Mixed batches of 4..256, beside against behind: 50 products 52 (84) us,
-// 1,000 116 (157), 5,000 244 (338), 20,000 654 (659), 35,000 1,111 (1,066),
-// 50,000 1,548 (1,488).
+// on.  Mixed batches of 4..256, beside against behind: 50 products 31 (44) us,
+// 1,000 82 (106), 5,000 177 (216), 20,000 604 (599), 35,000 1,035 (996),
+// 50,000 1,426 (1,384).
 constexpr unsigned FG_BESIDE = 20;
 constexpr unsigned FG_LONG = (1u << 28) - 1;  // products of a run an item word can hold
 
 // Plan: every run of entries sharing C becomes min(tiles, parts) items {first
 // entry, products << 4 | part}, counting-sorted heaviest first, in two lists:
 // C of more than 64 columns and 32 rows takes 64 x 128 tiles of 8 x 8 outputs
-// a thread, the rest 64 x 64 tiles of 8 x 4 or 4 x 4 (one list for all: 1.57 ms
-// on 50,000 products of 4..256, two lists 1.49 ms; one CTA a run on 64 x 64
-// tiles, as before: 4.66 ms).  The lists fill one array from its two ends.
+// a thread, the rest 64 x 64 tiles of 8 x 4 or 4 x 4 (one list for all took 1.57
+// ms on 50,000 products of 4..256 where two took 1.49, now 1.38; one CTA a run on
+// 64 x 64 tiles, as before: 4.66 ms).  The lists fill one array from its two ends.
 struct FlexPlan {
   unsigned *class_n, *class_fill;  // [2][FG_CLASSES]: small, wide
   unsigned *n_items, *counter;                 // [2]
@@ -80,6 +85,17 @@ __device__ __forceinline__ bool fg_wide(int M, int N) { return M > 32 && N > 64;
 __device__ __forceinline__ void fg_tiles(int M, int N, int *tiles_m, int *tiles_n) {
   *tiles_m = ceil_div(M, 64);
   *tiles_n = ceil_div(N, fg_wide(M, N) ? 128 : 64);
+}
+
+__device__ __forceinline__ FlexJob fg_job(const LibShalom_sgemm_entry &e, int N) {
+  FlexJob j;
+  j.A = e.A; j.B = e.B; j.C = e.C;
+  j.K = max(0, e.K); j.transb = e.transb;
+  j.lda = e.lda > 0 ? e.lda : j.K;
+  j.ldb = e.ldb > 0 ? e.ldb : (e.transb ? j.K : N);
+  j.ldc = e.ldc > 0 ? e.ldc : N;
+  j.alpha = e.alpha; j.beta = e.beta;
+  return j;
 }
 
 // items, class and length of the run starting at entry i (0 items: empty C)
@@ -162,6 +178,60 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// The lists of a batch of few products in one launch of one block: the memset
+// and the passes over the chip cost more than the kernels (256 products of 32^3:
+// 15.0 us with them, 10.2 with this).
+constexpr int PLAN_THREADS = 512, PLAN_EACH = 4;
+__global__ void __launch_bounds__(PLAN_THREADS)
+    k_fg_plan_one(const LibShalom_sgemm_entry *e, int count, FlexPlan pl) {
+  __shared__ unsigned n[2 * FG_CLASSES], sums[2 * FG_CLASSES / 32];
+  static_assert(FG_CLASSES == 64, "two warps a list");
+  chain_next();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid < 2 * FG_CLASSES) n[tid] = 0;
+  __syncthreads();
+  unsigned rank[PLAN_EACH], products[PLAN_EACH];
+  int cls[PLAN_EACH], parts[PLAN_EACH];
+#pragma unroll
+  for (int u = 0; u < PLAN_EACH; ++u) {
+    const int i = u * PLAN_THREADS + tid;
+    parts[u] = 0;
+    if (i >= count || (i > 0 && e[i].C == e[i - 1].C)) continue;
+    long len;
+    parts[u] = fg_run(e, count, i, pl.parts, &len, &cls[u]);
+    products[u] = (unsigned)len;
+    if (parts[u]) rank[u] = atomicAdd(&n[cls[u]], (unsigned)parts[u]);
+  }
+  __syncthreads();
+  // first slot of every class, heavy classes of a list first
+  const int at = (tid & ~(FG_CLASSES - 1)) + FG_CLASSES - 1 - (tid & (FG_CLASSES - 1));
+  const unsigned own = tid < 2 * FG_CLASSES ? n[at] : 0;
+  unsigned upto = own;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned v = __shfl_up_sync(0xffffffffu, upto, d);
+    if (lane >= d) upto += v;
+  }
+  if (tid < 2 * FG_CLASSES && lane == 31) sums[warp] = upto;
+  __syncthreads();
+  if (tid < 2 * FG_CLASSES) {
+    if (warp & 1) upto += sums[warp - 1];
+    n[at] = upto - own;
+    if ((warp & 1) && lane == 31) {
+      pl.n_items[warp >> 1] = upto;
+      pl.counter[warp >> 1] = 0;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < PLAN_EACH; ++u)
+    for (int p = 0; p < parts[u]; ++p) {
+      const long slot = (long)n[cls[u]] + rank[u] + p;
+      pl.items[cls[u] < FG_CLASSES ? slot : pl.n - 1 - slot] =
+          make_uint2((unsigned)(u * PLAN_THREADS + tid), products[u] << 4 | (unsigned)p);
+    }
+}
+
 // CTAs take items from a counter.  Thread 0 keeps two items ahead: the list
 // word of the next item and the counter value after it are in flight while an
 // item is computed (inline PTX: the compiler would aggregate an atomicAdd over
@@ -172,7 +242,13 @@ __global__ void __launch_bounds__(FX_THREADS, WIDE ? 4 : 6)
   extern __shared__ __align__(16) float fsm[];
   __shared__ uint2 s_item[2];
   if constexpr (WIDE) chain_wait();  // the plan
-  const unsigned n_items = pl.n_items[WIDE];
+  // Few small items: the four quarters of each 64 x 64 tile are items of their
+  // own (a tile's latency is what counts then; B200, 64 products of 64^3 17.5 ->
+  // 10.3 us, a run of 128 such products 914 -> 416, 64 of 64 x 64 x 5,000 405 ->
+  // 243).
+  const unsigned n_tiles = pl.n_items[WIDE];
+  const bool quarters = !WIDE && 4 * n_tiles <= gridDim.x;
+  const unsigned n_items = quarters ? 4 * n_tiles : n_tiles;
   // The small list's blocks may start when all of this kernel's have: the plan
   // is complete then, nothing that either writes is the other's, and the wait
   // at the end keeps what follows in the stream behind both.
@@ -185,12 +261,14 @@ __global__ void __launch_bounds__(FX_THREADS, WIDE ? 4 : 6)
                  : "l"(pl.counter + WIDE)
                  : "memory");
   };
-  auto at = [&](long i) { return pl.items[WIDE ? pl.n - 1 - i : i]; };
+  auto at = [&](long i) { return pl.items[WIDE ? pl.n - 1 - i : quarters ? i % n_tiles : i]; };
   if (threadIdx.x == 0) {
     s_item[0] = blockIdx.x < n_items ? at(blockIdx.x) : make_uint2(0, 0);
     const unsigned i1 = blockIdx.x + gridDim.x;
-    if (i1 < n_items) nxt = at(i1);
-    take();
+    if (i1 < n_items) {
+      nxt = at(i1);
+      take();
+    }
   }
   __syncthreads();
   for (int it = 0;; it ^= 1) {
@@ -214,19 +292,22 @@ __global__ void __launch_bounds__(FX_THREADS, WIDE ? 4 : 6)
     const int em = flex_edge(M, tiles_m), en = flex_edge(N, tiles_n);
     for (long t = item.y & (FG_PARTS - 1); t < (long)tiles_m * tiles_n; t += pl.parts) {
       const int tm = (int)(t / tiles_n), tn = (int)(t - (long)tm * tiles_n);
-      const int m0 = tm * em, n0 = tn * en, mrows = min(em, M - m0), ncols = min(en, N - n0);
+      int m0 = tm * em, n0 = tn * en, mrows = min(em, M - m0), ncols = min(en, N - n0);
+      if (quarters) {
+        const unsigned quarter = blockIdx.x / n_tiles;
+        const int dm = quarter & 2 ? 32 : 0, dn = quarter & 1 ? 32 : 0;
+        m0 += dm;
+        n0 += dn;
+        mrows = min(32, mrows - dm);
+        ncols = min(32, ncols - dn);
+      }
       if (mrows <= 0 || ncols <= 0) continue;
       const bool small = ((mrows + 3) >> 2) * ((ncols + 3) >> 2) <= FX_THREADS;
       for (long p = 0; p < len || (len == FG_LONG && p < most && run[p].C == run->C); ++p) {
-        const LibShalom_sgemm_entry &e = run[p];
-        FlexJob j;
-        j.A = e.A; j.B = e.B; j.C = e.C;
-        j.K = max(0, e.K); j.transb = e.transb;
-        j.lda = e.lda > 0 ? e.lda : j.K;
-        j.ldb = e.ldb > 0 ? e.ldb : (e.transb ? j.K : N);
-        j.ldc = e.ldc > 0 ? e.ldc : N;
-        j.alpha = e.alpha; j.beta = e.beta;
+        if (p + 1 < len) asm volatile("prefetch.global.L1 [%0];" ::"l"(run + p + 1));
+        const FlexJob j = fg_job(run[p], N);
         if constexpr (WIDE) flex_tile<F128, 8, 8>(j, m0, n0, mrows, ncols, fsm);
+        else if (quarters) flex_tile<F32, 4, 4>(j, m0, n0, mrows, ncols, fsm);
         else if (small) flex_tile<F64, 4, 4>(j, m0, n0, mrows, ncols, fsm);
         else flex_tile<F64, 8, 4>(j, m0, n0, mrows, ncols, fsm);
       }
@@ -234,6 +315,39 @@ __global__ void __launch_bounds__(FX_THREADS, WIDE ? 4 : 6)
     __syncthreads();
   }
   if constexpr (!WIDE) chain_wait();
+}
+
+// A batch of few products without lists: FG_PARTS blocks for each entry, which
+// deal the tiles of the run that starts there (64 x 128 tiles, or 32 x 32: a
+// tile's latency is what counts).  One launch and no scratch: 16 products of 8^3
+// 4.4 us, 8.2 with the plan and the list kernels.  More entries than the chip
+// holds sixteenfold leave its SMs unevenly loaded (64 products of 100^3: 38.9 us,
+// 22.5 with the lists).
+constexpr long FG_FEW = 32;
+__global__ void __launch_bounds__(FX_THREADS, 4)
+    k_flex_few(const LibShalom_sgemm_entry *entries, long count) {
+  extern __shared__ __align__(16) float fsm[];
+  for (long w = blockIdx.x; w < count * FG_PARTS; w += gridDim.x) {
+    const long part = w / count, i = w - part * count, most = count - i;
+    const LibShalom_sgemm_entry *run = entries + i;
+    if (i > 0 && run->C == run[-1].C) continue;
+    const int M = run->M, N = run->N;
+    if (M <= 0 || N <= 0) continue;
+    const bool wide = fg_wide(M, N);
+    const int tiles_m = ceil_div(M, wide ? 64 : 32), tiles_n = ceil_div(N, wide ? 128 : 32);
+    const int em = flex_edge(M, tiles_m), en = flex_edge(N, tiles_n);
+    for (long t = part; t < (long)tiles_m * tiles_n; t += FG_PARTS) {
+      const int tm = (int)(t / tiles_n), tn = (int)(t - (long)tm * tiles_n);
+      const int m0 = tm * em, n0 = tn * en, mrows = min(em, M - m0), ncols = min(en, N - n0);
+      if (mrows <= 0 || ncols <= 0) continue;
+      for (long p = 0; p < most && run[p].C == run->C; ++p) {
+        if (p + 1 < most) asm volatile("prefetch.global.L1 [%0];" ::"l"(run + p + 1));
+        const FlexJob j = fg_job(run[p], N);
+        if (wide) flex_tile<F128, 8, 8>(j, m0, n0, mrows, ncols, fsm);
+        else flex_tile<F32, 4, 4>(j, m0, n0, mrows, ncols, fsm);
+      }
+    }
+  }
 }
 
 template <class Cfg, int TM, int TN, int PER_SM>
@@ -265,8 +379,13 @@ int run_flex_strided(const GemmArgs<float> &g, long sA, long sB, long sC, long c
   u.alpha = g.alpha; u.beta = g.beta;
   // the smallest thread tile that covers a product in one CTA, 8 x 8 (fewest
   // shared-memory loads per FMA) beyond 64 columns.  B200, 10,000 products
-  // against the fixed 32 / 64 / 128 tiles before: 24^3 NN 49 (74) us, 33^3 NN 90
-  // (217), 64^3 NN 198 (213), 72^3 NT 495 (959), 104^3 NT 959 (1,241)
+  // against the fixed 32 / 64 / 128 tiles before: 24^3 NN 39 (74) us, 104^3 NT
+  // 895 (1,241); 3,000 of 64^3 NN 54 (70), of 8 x 100 x 64 40 (184), of 128 x 16 x
+  // 64 64 (205), of 300 x 33 x 50 193 (590); 222 of 256^3 177 (197), 16 of 512^3
+  // 115 (123)
+  // Few products: 32 x 32 tiles, whose latency is what counts.
+  if (cdiv(g.M, 32) * cdiv(g.N, 32) * count <= FU_FEW * (long)state().num_sms)
+    return launch_uniform<F32, 4, 4, 6>(u, count);
   if (cdiv(g.M, 4) * cdiv(g.N, 4) <= FX_THREADS && g.M <= 64 && g.N <= 64)
     return launch_uniform<F64, 4, 4, 6>(u, count);
   if (g.N <= 64) return launch_uniform<F64, 8, 4, 6>(u, count);
@@ -276,6 +395,13 @@ int run_flex_strided(const GemmArgs<float> &g, long sA, long sB, long sC, long c
 int run_grouped_s(const LibShalom_sgemm_entry *entries, long count) {
   State &st = state();
   if (count > UINT32_MAX) return LIBSHALOM_ERR_UNSUPPORTED;
+  if (count <= FG_FEW) {
+    const int per_sm = occupancy_of((const void *)k_flex_few, FX_THREADS, F128::SMEM, 4);
+    k_flex_few<<<grid_for(count * FG_PARTS, per_sm), FX_THREADS, F128::SMEM, st.stream>>>(entries,
+                                                                                         count);
+    LS_CUDA_TRY(cudaGetLastError());
+    return LIBSHALOM_SUCCESS;
+  }
   const size_t header = 512;
   FlexPlan pl;
   // one item a run where the items would take much memory
@@ -294,11 +420,16 @@ int run_grouped_s(const LibShalom_sgemm_entry *entries, long count) {
   pl.n_items = w + 4 * FG_CLASSES;
   pl.counter = pl.n_items + 2;
   pl.items = reinterpret_cast<uint2 *>(w + header);
-  LS_CUDA_TRY(cudaMemsetAsync(w, 0, header * sizeof(unsigned), st.stream));
-  const int pgrid = (int)std::max(1L, std::min(cdiv(count, 256), (long)st.num_sms * 8));
-  k_fg_count<<<pgrid, 256, 0, st.stream>>>(entries, count, pl);
-  LS_CUDA_TRY(cudaGetLastError());
-  if ((rc = launch_chained(k_fg_place, pgrid, 256, 0, st.stream, entries, count, pl))) return rc;
+  if (count <= PLAN_THREADS * PLAN_EACH) {
+    k_fg_plan_one<<<1, PLAN_THREADS, 0, st.stream>>>(entries, (int)count, pl);
+    LS_CUDA_TRY(cudaGetLastError());
+  } else {
+    LS_CUDA_TRY(cudaMemsetAsync(w, 0, header * sizeof(unsigned), st.stream));
+    const int pgrid = (int)std::max(1L, std::min(cdiv(count, 256), (long)st.num_sms * 8));
+    k_fg_count<<<pgrid, 256, 0, st.stream>>>(entries, count, pl);
+    LS_CUDA_TRY(cudaGetLastError());
+    if ((rc = launch_chained(k_fg_place, pgrid, 256, 0, st.stream, entries, count, pl))) return rc;
+  }
   const int ps_w = occupancy_of((const void *)k_flex_grouped<true>, FX_THREADS, F128::SMEM, 4);
   const int ps_s = occupancy_of((const void *)k_flex_grouped<false>, FX_THREADS, F64::SMEM, 6);
   rc = launch_chained(k_flex_grouped<true>, grid_for((long)st.num_sms * ps_w, ps_w), FX_THREADS,
