@@ -1201,7 +1201,12 @@ constexpr int GRP_CLASSES = 64;  // work classes (total K slabs of the run, capp
 // 352 against 502 us; 256^3 NT, 1,000: 463 against 584 us), but as a second
 // kernel it only pays when there are enough of them to fill the machine.
 // Small runs with a product of several K chunks that reads C have a list of their
-// own (HOLD).
+// own (HOLD).  Where all the small runs get an SM of their own, the long ones
+// (GRP_LONG slabs) go to k_tc_grouped as well: it keeps a run's products in a
+// pipeline, where a tile of the small-product kernel is a chain of latencies.
+// Runs of 16 products of 64^3 on 148 or fewer C: 88 against 122 to 144 us (222 C:
+// 152 against 156), of 4 products 37 against 40; of 16 products of 32^3 62 against
+// 69; of 16 products of 128^3 170 against 180 to 240.
 enum : int { GRP_SMALL = 0, GRP_HOLD = 1, GRP_LARGE = 2, GRP_LISTS = 3, GRP_EMPTY = 3 };
 constexpr int GRP_SMALL_EDGE = 256;
 constexpr int GRP_SMALL_TILES =
@@ -1211,21 +1216,28 @@ static_assert(GRP_SMALL_TILES <= 16 && GRP_HOLD == 1, "an item word holds four b
 
 // workspace layout of the plan (unsigned words)
 struct GrpPlan {
-  unsigned *class_n;     // [6][GRP_CLASSES] per class: items of the small and of the hold
+  unsigned *class_n;     // [7][GRP_CLASSES] per class: items of the small and of the hold
                          // runs, the large runs; then, of the runs that can be either, the
-                         // same items and the runs
+                         // same items and the runs; then all runs but the large ones
   unsigned *class_off;   // [3][GRP_CLASSES] first sorted slot of each class (lists by kind)
   unsigned *class_fill;  // [3][GRP_CLASSES] slots taken so far
   unsigned *n_items;     // [3] items of the small-product kernel, runs of k_tc_grouped
   unsigned *counter;     // [1] work counter of the small-product kernel
-  unsigned *either_large;  // [1] where the runs that can be either go
+  unsigned *to_large;      // [1] which small runs go to k_tc_grouped: those that can be
+                           // either (bit 0), the long ones (bit 1)
   unsigned either_min;     // runs that can be either for them to go to k_tc_grouped
+  unsigned long_max;       // runs, but the large ones, for the long ones to go there
   uint2 *items;          // [n_slots]: small upwards, hold downwards; null: every run is large
   long n_slots;          // GRP_SMALL_TILES * count
   unsigned *run_first;   // [count] first entry of the large run in sorted slot s
   unsigned *run_len;     // [count]
 };
+constexpr int GRP_COUNTS = 2 * GRP_LISTS + 1;
 constexpr int GRP_HEADER = 1024;  // words of the class tables and counts
+static_assert((GRP_COUNTS + 2 * GRP_LISTS) * GRP_CLASSES + 16 <= GRP_HEADER, "class tables");
+// class from which a run is long; C blocks of less than 32 x 32 stay below it
+// (64 products of 8^3 on 148 C: 159 us in the small-product kernel, 184 in the other)
+constexpr int GRP_LONG = 16;
 
 struct GrpArgs {
   const LibShalom_sgemm_entry *entries;
@@ -1271,7 +1283,7 @@ __device__ __forceinline__ int grp_run_class(const LibShalom_sgemm_entry *e, lon
           : hold                                        ? GRP_HOLD
                                                         : GRP_SMALL;
   *either = *either && (*kind == GRP_SMALL || *kind == GRP_HOLD);
-  return (int)min(k_slabs, (long)GRP_CLASSES - 1);
+  return (int)min(k_slabs, (long)M * N < 1024 ? GRP_LONG - 1L : GRP_CLASSES - 1L);
 }
 
 // pass 1: items per work class
@@ -1279,7 +1291,7 @@ __device__ __forceinline__ int grp_run_class(const LibShalom_sgemm_entry *e, lon
 // of the classes took 17 us on 50,000 products)
 __global__ void __launch_bounds__(256)
     k_grp_count(const LibShalom_sgemm_entry *e, long count, GrpPlan pl) {
-  constexpr int NC = 2 * GRP_LISTS * GRP_CLASSES;
+  constexpr int NC = GRP_COUNTS * GRP_CLASSES;
   __shared__ unsigned n[NC];
   chain_next();
   for (int c = threadIdx.x; c < NC; c += 256) n[c] = 0;
@@ -1294,6 +1306,7 @@ __global__ void __launch_bounds__(256)
     unsigned *at = n + cls + (either ? GRP_LISTS * GRP_CLASSES : 0);
     atomicAdd(at + kind * GRP_CLASSES, kind == GRP_LARGE ? 1u : (unsigned)tiles);
     if (either) atomicAdd(at + GRP_LARGE * GRP_CLASSES, 1u);
+    if (kind != GRP_LARGE) atomicAdd(n + 2 * GRP_LISTS * GRP_CLASSES + cls, 1u);
   }
   __syncthreads();
   for (int c = threadIdx.x; c < NC; c += 256)
@@ -1305,21 +1318,29 @@ __global__ void __launch_bounds__(256)
 constexpr int GRP_OFF_THREADS = GRP_LISTS * GRP_CLASSES;
 __global__ void __launch_bounds__(GRP_OFF_THREADS) k_grp_offsets(GrpPlan pl) {
   static_assert(GRP_CLASSES == 64, "two warps a list");
-  __shared__ unsigned either_runs[2], sums[2 * GRP_LISTS];
+  __shared__ unsigned either_runs[2], runs[2], sums[2 * GRP_LISTS];
   chain_wait();
   chain_next();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int l = tid / GRP_CLASSES, at = l * GRP_CLASSES + GRP_CLASSES - 1 - tid % GRP_CLASSES;
+  const int l = tid / GRP_CLASSES, c = GRP_CLASSES - 1 - tid % GRP_CLASSES;
+  const int at = l * GRP_CLASSES + c;
   unsigned own = pl.class_n[at];
   const unsigned either = pl.class_n[GRP_LISTS * GRP_CLASSES + at];
+  const unsigned other = pl.class_n[2 * GRP_LISTS * GRP_CLASSES + c];
   if (l == GRP_LARGE) {
-    const unsigned runs = __reduce_add_sync(0xffffffffu, either);
-    if (lane == 0) either_runs[warp & 1] = runs;
+    const unsigned e = __reduce_add_sync(0xffffffffu, either);
+    const unsigned r = __reduce_add_sync(0xffffffffu, other);
+    if (lane == 0) {
+      either_runs[warp & 1] = e;
+      runs[warp & 1] = r;
+    }
   }
   __syncthreads();
-  const bool large = either_runs[0] + either_runs[1] >= pl.either_min;
-  if (tid == 0) *pl.either_large = large;
-  if ((l == GRP_LARGE) == large) own += either;
+  const bool either_large = either_runs[0] + either_runs[1] >= pl.either_min;
+  const bool long_large = !either_large && runs[0] + runs[1] <= pl.long_max;
+  if (tid == 0) *pl.to_large = (either_large ? 1u : 0u) | (long_large ? 2u : 0u);
+  if ((l == GRP_LARGE) == either_large) own += either;
+  if (long_large && c >= GRP_LONG) own = l == GRP_LARGE ? own + other : 0;
   unsigned upto = own;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
@@ -1341,7 +1362,7 @@ __global__ void __launch_bounds__(256)
   __shared__ unsigned n[NC], base[NC];
   chain_wait();
   chain_next();
-  const bool either_large = *pl.either_large != 0;
+  const unsigned to_large = *pl.to_large;
   const int tid = threadIdx.x;
   for (long i0 = blockIdx.x * 256L; i0 < count; i0 += gridDim.x * 256L) {
     if (tid < NC) n[tid] = 0;
@@ -1352,7 +1373,9 @@ __global__ void __launch_bounds__(256)
     bool either;
     if (i < count && grp_run_start(e, i)) {
       cls = grp_run_class(e, count, i, pl.items != nullptr, &len, &kind, &tiles, &either);
-      if (either && either_large) kind = GRP_LARGE;
+      if (kind != GRP_EMPTY &&
+          ((either && (to_large & 1)) || (cls >= GRP_LONG && (to_large & 2))))
+        kind = GRP_LARGE;
       cls += kind * GRP_CLASSES;
     }
     const unsigned rank =
@@ -2225,12 +2248,13 @@ int tc_sgemm_grouped(const LibShalom_sgemm_entry *entries, long count, int mode)
   unsigned *w = static_cast<unsigned *>(ws);
   GrpPlan pl;
   pl.class_n = w;
-  pl.class_off = pl.class_n + 2 * GRP_LISTS * GRP_CLASSES;
+  pl.class_off = pl.class_n + GRP_COUNTS * GRP_CLASSES;
   pl.class_fill = pl.class_off + GRP_LISTS * GRP_CLASSES;
   pl.n_items = pl.class_fill + GRP_LISTS * GRP_CLASSES;
   pl.counter = pl.n_items + GRP_LISTS;
-  pl.either_large = pl.counter + 1;
+  pl.to_large = pl.counter + 1;
   pl.either_min = 2u * (unsigned)st.num_sms;
+  pl.long_max = (unsigned)st.num_sms;
   pl.items = with_small ? reinterpret_cast<uint2 *>(w + GRP_HEADER) : nullptr;
   pl.n_slots = (long)GRP_SMALL_TILES * count;
   pl.run_first = w + GRP_HEADER + (with_small ? item_words : 0);
