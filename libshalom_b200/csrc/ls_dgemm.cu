@@ -65,10 +65,17 @@ __device__ __forceinline__ bool run_start(const LibShalom_dgemm_entry *e, long i
 // run starting at entry i: length, and its bin (shape, cost class: operand
 // doubles / 256, capped; heavy classes first), or -1 for a C block above 32 x 32.
 // Four entries are read at a time: a run's length is a chain of loads.
+// Deep runs: where every run has an SM of its own, a run of k_dgemm_small_runs
+// takes about 1.8 us for 16 k of a product and one of k_dgemm_runs 3.1 us for
+// 32 k (one run of 64 products of 32^3 240 against 209 us, with K = 16 129 against
+// 176, with K = 48 348 against 368; a product of 32 x 32 x 512 61 against 55).
+// With 148 runs the two are equal, with more the small kernel is faster.  (The
+// first product's K stands for the run's.)
 __device__ __forceinline__ int run_bin(const LibShalom_dgemm_entry *e, long count, long i,
                                        long *len) {
   const int M = e[i].M, N = e[i].N;
   const double *C = e[i].C;
+  const long s16 = (max(0, e[i].K) + 15L) >> 4, s32 = (max(0, e[i].K) + 31L) >> 5;
   long cost = (long)M * N, j = i;
   for (bool in = true; in;) {
     const double *c[4];
@@ -91,7 +98,9 @@ __device__ __forceinline__ int run_bin(const LibShalom_dgemm_entry *e, long coun
   *len = j - i;
   if (M > 32 || N > 32) return -1;
   const int shape = M <= 16 ? 2 : N <= 16 ? 1 : 0;
-  return shape * DM_CLASSES + DM_CLASSES - 1 - (int)max(0L, min(cost / 256, (long)DM_CLASSES - 1));
+  const bool deep = *len * s16 >= 32 && 7 * s16 > 12 * s32;
+  const long cls = deep ? DM_CLASSES - 1 : max(0L, min(cost / 256, DM_CLASSES - 2L));
+  return shape * DM_CLASSES + DM_CLASSES - 1 - (int)cls;
 }
 
 // Runs are counted per block in shared memory first: thousands of atomics on
@@ -121,9 +130,14 @@ __global__ void __launch_bounds__(256)
     atomicAdd(&pl.bin_runs[threadIdx.x], n[threadIdx.x]);
 }
 
-// off[b]: runs in the bins before b (own: thread b's bin); n_shape: their sums
-__device__ __forceinline__ void bin_offsets(unsigned own, unsigned *off, unsigned *n_shape) {
-  __shared__ unsigned sums[DM_BINS / 32];
+// bins of the deep runs: the first of each shape
+__device__ __forceinline__ bool deep_bin(int bin) { return bin < DM_BINS && bin % DM_CLASSES == 0; }
+
+// off[b]: runs in the bins before b (own: thread b's bin); n_shape: their sums.
+// Returns whether the deep ones are left out: there are no more than `few` runs.
+__device__ __forceinline__ bool bin_offsets(unsigned own, unsigned few, unsigned *off,
+                                            unsigned *n_shape) {
+  __shared__ unsigned sums[DM_BINS / 32], deep[DM_SHAPES];
   static_assert(DM_BINS <= 256 && DM_BINS % 32 == 0 && DM_CLASSES % 32 == 0, "one thread a bin");
   const int tid = threadIdx.x, lane = tid & 31;
   unsigned upto = own;
@@ -133,16 +147,27 @@ __device__ __forceinline__ void bin_offsets(unsigned own, unsigned *off, unsigne
     if (lane >= s) upto += v;
   }
   if (tid < DM_BINS && lane == 31) sums[tid >> 5] = upto;
+  if (deep_bin(tid)) deep[tid / DM_CLASSES] = own;
   __syncthreads();
+  bool leave_out = false;
+  if (deep[0] | deep[1] | deep[2]) {
+    unsigned all = 0;
+#pragma unroll
+    for (int i = 0; i < DM_BINS / 32; ++i) all += sums[i];
+    leave_out = all <= few;
+  }
   if (tid < DM_BINS) {
     for (int i = 0; i < tid >> 5; ++i) upto += sums[i];
+    if (leave_out)
+      for (int s = 0; s <= tid / DM_CLASSES; ++s) upto -= deep[s];
     off[tid] = upto - own;
   }
   if (n_shape && tid < DM_SHAPES) {
-    unsigned runs = 0;
+    unsigned runs = leave_out ? 0u - deep[tid] : 0u;
     for (int i = 0; i < DM_CLASSES / 32; ++i) runs += sums[tid * (DM_CLASSES / 32) + i];
     n_shape[tid] = runs;
   }
+  return leave_out;
 }
 
 // Every block sums the bins itself (192 words, two shuffled scans): a launch
@@ -153,12 +178,19 @@ __global__ void __launch_bounds__(256)
   chain_wait();
   chain_next();
   const int tid = threadIdx.x;
-  bin_offsets(tid < DM_BINS ? pl.bin_runs[tid] : 0, off, blockIdx.x == 0 ? pl.n_shape : nullptr);
+  const bool leave_out = bin_offsets(tid < DM_BINS ? pl.bin_runs[tid] : 0, pl.few, off,
+                                     blockIdx.x == 0 ? pl.n_shape : nullptr);
   for (long i0 = blockIdx.x * 256L; i0 < count; i0 += gridDim.x * 256L) {
     if (tid < DM_BINS) n[tid] = 0;
     __syncthreads();
     const long i = i0 + tid;
-    const int bin = i < count ? pl.entry_bin[i] : DM_BINS;
+    int bin = i < count ? pl.entry_bin[i] : DM_BINS;
+    if (leave_out && deep_bin(bin)) {
+      const unsigned slot = atomicAdd(pl.n_large, 1u);
+      pl.large_first[slot] = (unsigned)i;
+      pl.large_len[slot] = pl.entry_len[i];
+      bin = DM_BINS;
+    }
     unsigned rank = 0;
     if (bin < DM_BINS) rank = atomicAdd(&n[bin], 1u);
     __syncthreads();
@@ -204,9 +236,18 @@ __global__ void __launch_bounds__(PLAN_ONE_THREADS)
     }
   }
   __syncthreads();
-  if (tid == 0) *pl.n_large = large;
-  bin_offsets(tid < DM_BINS ? n[tid] : 0, off, pl.n_shape);
+  if (bin_offsets(tid < DM_BINS ? n[tid] : 0, pl.few, off, pl.n_shape)) {
+#pragma unroll
+    for (int u = 0; u < PLAN_ONE_EACH; ++u) {
+      if (!deep_bin(bin[u])) continue;
+      const unsigned slot = atomicAdd(&large, 1u);
+      pl.large_first[slot] = (unsigned)(u * PLAN_ONE_THREADS + tid);
+      pl.large_len[slot] = length[u];
+      bin[u] = DM_BINS;
+    }
+  }
   __syncthreads();
+  if (tid == 0) *pl.n_large = large;
 #pragma unroll
   for (int u = 0; u < PLAN_ONE_EACH; ++u) {
     if (bin[u] == DM_BINS) continue;
@@ -613,7 +654,7 @@ __global__ void __launch_bounds__(DR_THREADS, 6)
 
 }  // namespace
 
-int plan_dgemm_runs(const LibShalom_dgemm_entry *entries, long count, RunPlan *out) {
+int plan_dgemm_runs(const LibShalom_dgemm_entry *entries, long count, unsigned few, RunPlan *out) {
   State &st = state();
   if (count > (1L << 30)) return LIBSHALOM_ERR_UNSUPPORTED;
   const size_t header = 512;
@@ -623,6 +664,7 @@ int plan_dgemm_runs(const LibShalom_dgemm_entry *entries, long count, RunPlan *o
   if (rc) return rc;
   unsigned *w = static_cast<unsigned *>(ws);
   RunPlan pl;
+  pl.few = few;
   pl.n_large = w;
   pl.n_shape = w + 8;
   pl.bin_runs = w + 64;
@@ -651,7 +693,7 @@ int plan_dgemm_runs(const LibShalom_dgemm_entry *entries, long count, RunPlan *o
 // Grouped FP64 batch on the CUDA cores.
 int run_dgemm_runs(const LibShalom_dgemm_entry *entries, long count) {
   RunPlan pl;
-  int rc = plan_dgemm_runs(entries, count, &pl);
+  int rc = plan_dgemm_runs(entries, count, (unsigned)state().num_sms / 2, &pl);
   if (rc) return rc;
   const int per_sm = occupancy_of((const void *)k_dgemm_small_runs, DS_WARPS * 32, 0, DS_PER_SM);
   rc = launch_chained(k_dgemm_small_runs, grid_for(cdiv(2 * count, DS_WARPS), per_sm),

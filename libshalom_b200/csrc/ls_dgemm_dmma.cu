@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(DM_WARPS * 32, DM_PER_SM)
 
 int run_dgemm_dmma(const LibShalom_dgemm_entry *entries, long count) {
   RunPlan pl;
-  int rc = plan_dgemm_runs(entries, count, &pl);
+  int rc = plan_dgemm_runs(entries, count, 0, &pl);
   if (rc) return rc;
   const int per_sm = occupancy_of((const void *)k_dgemm_dmma, DM_WARPS * 32, 0, DM_PER_SM);
   rc = launch_chained(k_dgemm_dmma, grid_for(cdiv(count, DM_WARPS), per_sm), DM_WARPS * 32, 0,
