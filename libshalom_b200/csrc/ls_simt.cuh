@@ -238,10 +238,19 @@ __device__ __forceinline__ void simt_tile_impl(const GemmArgs<T> &g, long m0, lo
     }
     const T *as = smem + (s % STAGES) * Cfg::STAGE_ELEMS;
     const T *bs = as + Cfg::A_ELEMS;
-    // four of a slab's eight steps at a time: more loads ahead of the FMAs than
-    // with two (FP32 32 x 20480 x 4096: 201 -> 192 us, 1000^3 NT 102 -> 96),
-    // where all eight take 230 registers a thread and a CTA an SM less (222 us)
-#pragma unroll 4
+    // Four of a slab's eight steps at a time: more loads ahead of the FMAs than
+    // with two (FP32 32 x 20480 x 4096: 201 -> 192 us), where all eight take 230
+    // registers a thread and a CTA an SM less (222 us).  With op(B) = B^T four
+    // steps push some tiles past 128 registers, which is a CTA an SM less as well,
+    // and two are faster there: 2 x 2 outputs a thread (FP64 2048^3 2,113 us
+    // against 2,721, FP32 512^3 22.5 against 26.6), FP32 4 x 4 on 64 x 64 and 32 x
+    // 128 tiles without the GEMM_K blocks (32 x 20480 x 1024 90 against 102); and
+    // 4 x 8 is 4 % faster with two.
+    constexpr bool TWO = !TA && TB && (TM == 2 || (TM == 4 && TN == 8) ||
+                                       (sizeof(T) == 4 && KBLOCK == 0 && TM == 4 && TN == 4 &&
+                                        Cfg::BM <= 64));
+    constexpr int STEPS = TWO ? 2 : 4;
+#pragma unroll STEPS
     for (int kq = 0; kq < BK / EPU; ++kq) {
       // EPU consecutive k: a[i][t] = op(A)[row_i][k + t], b[t][j] = op(B)[k + t][col_j]
       T a[TM][EPU], b[EPU][TN];
