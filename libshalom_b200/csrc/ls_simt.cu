@@ -128,6 +128,12 @@ static int launch_single_l(const GemmArgs<T> &g, int splits, long kchunk,
                            T *partial, int ways_m, int ways_n, int per_sm) {
   const int tiles_m = (int)cdiv(g.M, Cfg::BM), tiles_n = (int)cdiv(g.N, Cfg::BN);
   const long items = (long)tiles_m * tiles_n * splits;
+  if constexpr (simt_two_steps<T, Cfg, KBLOCK, TA, TB>() && Cfg::TN <= 4) {
+    using Few = SimtCfg<T, Cfg::BM, Cfg::BN, Cfg::TM, Cfg::TN, true>;
+    if (items <= state().num_sms)
+      return launch_single_l<T, Few, KBLOCK, TA, TB>(g, splits, kchunk, partial, ways_m, ways_n,
+                                                     per_sm);
+  }
   const size_t smem = smem_of<T, Cfg>();
   auto kern = k_gemm_single<T, Cfg, KBLOCK, TA, TB>;
   per_sm = occupancy_of((const void *)kern, Cfg::NTH, smem, per_sm);
