@@ -41,11 +41,11 @@ struct GemmArgs {
   T alpha, beta;
 };
 
-// FEW: for products of so few tiles that no two share an SM (see STEPS)
-template <typename T, int BM_, int BN_, int TM_, int TN_, bool FEW_ = false>
+// FOUR: four steps unrolled, whatever that costs (see STEPS)
+template <typename T, int BM_, int BN_, int TM_, int TN_, bool FOUR_ = false>
 struct SimtCfg {
   static constexpr int BM = BM_, BN = BN_, TM = TM_, TN = TN_;
-  static constexpr bool FEW = FEW_;
+  static constexpr bool FOUR = FOUR_;
   // K per slab: one 128-byte shared-memory row of k (32 floats, 16 doubles)
   static constexpr int BK = 128 / (int)sizeof(T);
   static constexpr int EPU = 16 / (int)sizeof(T);  // elements per 16-byte unit
@@ -66,9 +66,10 @@ struct SimtCfg {
 template <typename T, class Cfg, int KBLOCK, bool TA, bool TB>
 constexpr bool simt_two_steps() {
   constexpr int TM = Cfg::TM, TN = Cfg::TN;
-  return !TA && TB && !Cfg::FEW &&
+  return !TA && TB && !Cfg::FOUR &&
          (TM == 2 || (TM == 4 && TN == 8) ||
-          (sizeof(T) == 4 && KBLOCK == 0 && TM == 4 && TN == 4 && Cfg::BM <= 64));
+          (sizeof(T) == 4 && KBLOCK == 0 && TM == 4 && TN == 4 && Cfg::BM <= 64) ||
+          (sizeof(T) == 8 && Cfg::BM == 64 && Cfg::BN == 64));
 }
 
 // vector read of R consecutive elements from shared memory
@@ -256,8 +257,7 @@ __device__ __forceinline__ void simt_tile_impl(const GemmArgs<T> &g, long m0, lo
     // and two are faster there: 2 x 2 outputs a thread (FP64 2048^3 2,113 us
     // against 2,721, FP32 512^3 22.5 against 26.6), FP32 4 x 4 on 64 x 64 and 32 x
     // 128 tiles without the GEMM_K blocks (32 x 20480 x 1024 90 against 102); and
-    // 4 x 8 is 4 % faster with two.  Where every tile has an SM of its own, four
-    // are faster for all but that one (256 x 256 x 1000 NT 26.6 against 28.7).
+    // 4 x 8 (FP32) and 64 x 64 (FP64) are 4 and 2 % faster with two.
     constexpr int STEPS = simt_two_steps<T, Cfg, KBLOCK, TA, TB>() ? 2 : 4;
 #pragma unroll STEPS
     for (int kq = 0; kq < BK / EPU; ++kq) {
