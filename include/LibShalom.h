@@ -157,8 +157,9 @@ LIBSHALOM_API int LibShalom_get_plan(int *tile_config, int *splits, int *table_e
 /* Operand staging of the tensor-core kernels: 1 (default) = TMA
  * (cp.async.bulk.tensor) with warp-specialized producer / converter / MMA /
  * epilogue warps whenever the operands are 16-byte aligned with 16-byte row
- * strides; 0 = always the cp.async kernel (any alignment).  Results are the
- * same either way. */
+ * strides; 0 = always the cp.async kernel (any alignment).  Results agree to
+ * rounding, bit for bit except for long K on tiles of at most 64 columns, whose
+ * kernel adds the correction products in another order. */
 LIBSHALOM_API int LibShalom_set_tma(int enable);
 
 /* Self-check of failure detection (no counterpart in the reference).  Every
@@ -211,8 +212,13 @@ typedef struct LibShalom_dgemm_entry {
 
 /* Grouped SGEMM over `count` entries that live in DEVICE memory.  Entries
  * are independent unless they name the same C; entries that share a C must
- * be contiguous in the array, have the same M and N, and are applied in
- * array order by one CTA. */
+ * be contiguous in the array, have the same M and N, and are applied in array
+ * order to each element of C.  Tiles of one C may be computed at the same time,
+ * so no A or B of the batch may overlap a C of it.
+ * The library keeps scratch for the largest call so far until
+ * LibShalom_finalize: 128 bytes an entry in plain FP32 (nothing up to 32
+ * entries, 8 bytes an entry beyond 4 Mi), 136 in the split-BF16 modes (8 beyond
+ * 16 Mi or where that cannot be had), 21 for LibShalom_dgemm_batched. */
 LIBSHALOM_API int LibShalom_sgemm_batched(const LibShalom_sgemm_entry *entries, long count);
 
 /* Uniform batch: count GEMMs of one shape, matrix g at A + g*strideA etc. */
@@ -259,9 +265,8 @@ LIBSHALOM_API int LibShalom_sgemm_batched_strided_host(int transb, long M, long 
  * reads a matrix a pending call writes, writes one a pending call reads, or
  * writes a pending call's C other than the directly preceding call's (same M
  * and N) first flushes the pending calls, and calls that cannot be recorded
- * (transa == Trans, or M N K above 128^3: the grouped kernels give each call
- * to one CTA, so larger calls run faster directly) flush and then run
- * directly; matrices
+ * (transa == Trans, or M N K above 128^3: larger calls fill the GPU on their
+ * own and run faster directly) flush and then run directly; matrices
  * that overlap without sharing a base pointer are the caller's to keep
  * apart.  Every other call that launches work (the batched, _ex, _host,
  * stack, convolution and no-allocation calls) launches the pending calls
@@ -305,8 +310,8 @@ LIBSHALOM_API int LibShalom_dgemm_ex(int transa, int transb, long M, long N, lon
                                      double alpha, const double *A, long lda, const double *B,
                                      long ldb, double beta, double *C, long ldc);
 
-/* Grouped DGEMM (same rules as LibShalom_sgemm_batched).  Arithmetic set by
- * LibShalom_set_dgemm_method. */
+/* Grouped DGEMM (same rules as LibShalom_sgemm_batched; C of a run has its first
+ * entry's ldc).  Arithmetic set by LibShalom_set_dgemm_method. */
 LIBSHALOM_API int LibShalom_dgemm_batched(const LibShalom_dgemm_entry *entries, long count);
 
 /* Stack front end (no counterpart in the reference): a batch described the

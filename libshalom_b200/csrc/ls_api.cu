@@ -621,8 +621,8 @@ int flush_deferred() {
   return rc;
 }
 
-// Largest call worth recording (M N K): the grouped kernels give each call to
-// one CTA, so a larger call runs faster directly, over many CTAs.
+// Largest call worth recording (M N K): a larger one fills the GPU on its own and
+// runs faster directly.
 constexpr double DEFER_MAX_MNK = 2097152.0;  // 128^3
 
 // Records a drop-in call while deferring.  Returns 1 when the call was

@@ -1190,14 +1190,16 @@ __global__ void __launch_bounds__(WsRoles<WIDE, (BLX == 1)>::THREADS, 1)
 // persistent CTAs take the sorted runs round-robin.  Inside a CTA a scheduler
 // warp expands its runs into (tile, product) items for the other roles.  The
 // products of a run are applied in array order by the one CTA that owns the
-// run (C = alpha_p A_p op(B_p) + beta_p C, product by product).
+// run (C = alpha_p A_p op(B_p) + beta_p C, product by product); in the
+// small-product kernel, by the one CTA that owns the tile.
 // ===========================================================================
 constexpr int GRP_CLASSES = 64;  // work classes (total K slabs of the run, capped)
 
-// Plan of a grouped batch.  Runs whose C is at most 256 x 256 become one item
-// per tile of the small-product kernel; larger runs go to k_tc_grouped, one
-// item per run.  Runs of full tiles with 16-byte aligned operands can go to
-// either: k_tc_grouped is faster on them (128 x 128 x 512 NT, 1,500 products:
+// Plan of a grouped batch.  Runs whose C is at most 256 x 256 (the largest that was
+// measured, not where the kernels meet) become one item per tile of the
+// small-product kernel; larger runs go to k_tc_grouped, one item per run.  Runs
+// of full tiles with 16-byte aligned operands can go to either: k_tc_grouped is
+// faster on them (128 x 128 x 512 NT, 1,500 products:
 // 352 against 502 us; 256^3 NT, 1,000: 463 against 584 us), but as a second
 // kernel it only pays when there are enough of them to fill the machine.
 // Small runs with a product of several K chunks that reads C have a list of their
@@ -2051,6 +2053,12 @@ int tc_launch(TcProblem &p, int mode) {
   memset(&mc, 0, sizeof(mc));
   WsArgs wa;
   const bool tma = st.use_tma && ws_maps(p, &ma, &mb, &mc, &wa);
+  // Rows that TMA cannot address: the small-product kernel at every size and K,
+  // single products included (against k_tc_sgemm, bf16x6: 10,000 of 45 x 37 x 51
+  // 96 us (456), 2,000 of 129^3 387 (2,006), 10 of 1001^3 345 (905), one of 257^3
+  // 25 (57), of 1001^3 94 (184), of 4095^3 1,904 (4,818), of 33 x 33 x 20481 948
+  // (3,794); beta = 1: 5,000 of 45 x 37 x 257 311 (1,077), 100 of 513^3 646
+  // (1,898)).  Split-K slices stay with k_tc_sgemm.
   if (!tma && st.use_tma && !p.kslice && p.lda < (1 << 30) && p.ldb < (1 << 30)) {
     TcSmallArgs sa{};
     sa.A = p.A; sa.B = p.B; sa.C = p.C;

@@ -221,7 +221,8 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
 }
 
 // Instruction descriptor of tcgen05.mma kind::f16: D f32, A and B bf16, both
-// K-major, M = 128, N = n (multiple of 16, <= 256).
+// K-major; M = 128 with N a multiple of 16, or M = 64 with N a multiple of 8 (N <=
+// 256).
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n) {
   return (1u << 4)                        // D format f32
          | (1u << 7)                      // A format bf16
