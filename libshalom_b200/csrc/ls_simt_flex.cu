@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(FX_THREADS, WIDE ? 4 : 6)
   // 10.3 us, a run of 128 such products 914 -> 416, 64 of 64 x 64 x 5,000 405 ->
   // 243).
   const unsigned n_tiles = pl.n_items[WIDE];
-  const bool quarters = !WIDE && 4 * n_tiles <= gridDim.x;
+  const bool quarters = !WIDE && n_tiles <= gridDim.x / 4;
   const unsigned n_items = quarters ? 4 * n_tiles : n_tiles;
   // The small list's blocks may start when all of this kernel's have: the plan
   // is complete then, nothing that either writes is the other's, and the wait
