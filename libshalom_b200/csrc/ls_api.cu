@@ -69,47 +69,57 @@ static bool caller_captures() {
   return status == cudaStreamCaptureStatusActive;
 }
 
-// A buffer that a caller's graph names is kept until finalize when it is
-// outgrown (each at most half as large as the next: together less than the one
-// in use); one that no graph names is freed once the stream is done with it.
-int workspace(size_t bytes, void **out) {
+// A buffer of at least `bytes` bytes, grown on demand.  One that a caller's graph
+// names is kept until finalize when it is outgrown (each at most half as large
+// as the next: together less than the one in use); one that no graph names is
+// freed once the stream is done with it.
+static int grow(DeviceBuffer &b, size_t bytes, void **out) {
   State &st = state();
   if (bytes < 256) bytes = 256;
   const bool captured = caller_captures();
-  if (st.ws && st.ws_bytes >= bytes && st.ws_device == st.device) {
-    st.ws_in_graph = st.ws_in_graph || captured;
-    *out = st.ws;
+  if (b.p && b.bytes >= bytes && b.device == st.device) {
+    b.in_graph = b.in_graph || captured;
+    *out = b.p;
     return LIBSHALOM_SUCCESS;
   }
   size_t want = std::max(bytes, (size_t)1 << 20);
-  if (st.ws && (st.ws_in_graph || captured || st.own_capture)) {
+  if (b.p && (b.in_graph || captured || st.own_capture)) {
     // (the stream cannot be waited for while it is captured)
-    want = std::max(want, 2 * st.ws_bytes);
-    st.ws_kept.push_back(st.ws);
-  } else if (st.ws) {
+    want = std::max(want, 2 * b.bytes);
+    st.kept.push_back(b.p);
+  } else if (b.p) {
     // kernels queued earlier may still read the old buffer
     LS_CUDA_TRY(cudaStreamSynchronize(st.stream));
-    cudaFree(st.ws);
+    cudaFree(b.p);
   }
-  st.ws = nullptr;
-  st.ws_bytes = 0;
+  b = DeviceBuffer();
   // cudaMalloc is no stream operation: the relaxed mode allows it in a capture
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   LS_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
-  const cudaError_t e = cudaMalloc(&st.ws, want);
+  const cudaError_t e = cudaMalloc(&b.p, want);
   LS_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
   if (e != cudaSuccess) {
     cudaGetLastError();
-    st.ws = nullptr;
+    b.p = nullptr;
     return LIBSHALOM_ERR_ALLOC;
   }
-  st.ws_in_graph = captured;
-  st.ws_bytes = want;
-  st.ws_device = st.device;
-  ++st.ws_generation;  // graphs captured with the old buffer are stale
-  *out = st.ws;
+  b.in_graph = captured;
+  b.bytes = want;
+  b.device = st.device;
+  *out = b.p;
   return LIBSHALOM_SUCCESS;
 }
+
+int workspace(size_t bytes, void **out) {
+  State &st = state();
+  const void *before = st.ws.p;
+  const int rc = grow(st.ws, bytes, out);
+  if (st.ws.p != before) ++st.ws_generation;  // graphs captured with the old buffer are stale
+  return rc;
+}
+
+// Buffer of the front ends.
+static int frontend_buffer(size_t bytes, void **out) { return grow(state().fe, bytes, out); }
 
 int grid_for(long work_items, int per_sm) {
   State &st = state();
@@ -155,32 +165,6 @@ int finish_launch(const char *what) {
       return LIBSHALOM_ERR_CUDA;
     }
   }
-  return LIBSHALOM_SUCCESS;
-}
-
-// Buffer of the front ends (grown on demand like the workspace).
-static int frontend_buffer(size_t bytes, void **out) {
-  State &st = state();
-  if (bytes < 256) bytes = 256;
-  if (st.fe && st.fe_bytes >= bytes && st.fe_device == st.device) {
-    *out = st.fe;
-    return LIBSHALOM_SUCCESS;
-  }
-  if (st.fe) {
-    LS_CUDA_TRY(cudaStreamSynchronize(st.stream));
-    cudaFree(st.fe);
-    st.fe = nullptr;
-    st.fe_bytes = 0;
-  }
-  const size_t want = std::max(bytes, (size_t)1 << 20);
-  if (cudaMalloc(&st.fe, want) != cudaSuccess) {
-    cudaGetLastError();
-    st.fe = nullptr;
-    return LIBSHALOM_ERR_ALLOC;
-  }
-  st.fe_bytes = want;
-  st.fe_device = st.device;
-  *out = st.fe;
   return LIBSHALOM_SUCCESS;
 }
 
@@ -840,7 +824,7 @@ int LibShalom_set_stream(void *stream) {
     // before calls on the new stream can overwrite them.  (A stream the
     // caller has already destroyed reports an error here, which is ignored:
     // its queued work completes anyway.)
-    if (st.ws || st.fe) {
+    if (st.ws.p || st.fe.p) {
       if (cudaStreamSynchronize(st.stream) != cudaSuccess) cudaGetLastError();
     }
     st.stream = next;
@@ -951,7 +935,7 @@ void LibShalom_finalize(void) {
   State &st = state();
   // calls still pending in a deferred section run before anything is freed
   const int flushed = flush_deferred();
-  if (st.ws || st.fe || !st.ws_kept.empty()) cudaStreamSynchronize(st.stream);
+  if (st.ws.p || st.fe.p || !st.kept.empty()) cudaStreamSynchronize(st.stream);
   graph_cache_clear();
   if (st.ring_busy && st.ring_ev) cudaEventSynchronize(st.ring_ev);
   if (st.ring_ev) cudaEventDestroy(st.ring_ev);
@@ -971,17 +955,12 @@ void LibShalom_finalize(void) {
     host_staging_release();
     if (cur >= 0) cudaSetDevice(cur);
   }
-  if (st.ws) cudaFree(st.ws);
-  for (void *p : st.ws_kept) cudaFree(p);
-  st.ws_kept.clear();
-  st.ws_in_graph = false;
-  if (st.fe) cudaFree(st.fe);
-  st.ws = nullptr;
-  st.ws_bytes = 0;
-  st.ws_device = -1;
-  st.fe = nullptr;
-  st.fe_bytes = 0;
-  st.fe_device = -1;
+  for (DeviceBuffer *b : {&st.ws, &st.fe}) {
+    if (b->p) cudaFree(b->p);
+    *b = DeviceBuffer();
+  }
+  for (void *p : st.kept) cudaFree(p);
+  st.kept.clear();
   st.ring_device = -1;
   set_error(flushed);
 }

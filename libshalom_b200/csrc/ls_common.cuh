@@ -34,6 +34,13 @@ void note_cuda_error(cudaError_t e, const char *what, const char *file,
 // ---------------------------------------------------------------------------
 // library state (one instance per process; guarded by mu)
 // ---------------------------------------------------------------------------
+struct DeviceBuffer {
+  void *p = nullptr;
+  size_t bytes = 0;
+  int device = -1;
+  bool in_graph = false;  // a caller's graph names it
+};
+
 struct State {
   std::mutex mu;
   int device = -1;
@@ -55,17 +62,12 @@ struct State {
   // allow it (LIBSHALOM_NO_TMA=1 in the environment selects the cp.async one)
   bool use_tma = true;
   // device workspace (split-K partials, work counters, work lists)
-  void *ws = nullptr;
-  size_t ws_bytes = 0;
-  int ws_device = -1;
-  bool ws_in_graph = false;     // a caller's graph names the workspace
-  std::vector<void *> ws_kept;  // outgrown workspaces that callers' graphs name
-  bool own_capture = false;     // the graph cache is capturing
+  DeviceBuffer ws;
   // front-end buffer (stack entries, im2col columns): separate from the
   // workspace, which the GEMM paths the front ends call use themselves
-  void *fe = nullptr;
-  size_t fe_bytes = 0;
-  int fe_device = -1;
+  DeviceBuffer fe;
+  std::vector<void *> kept;  // outgrown buffers that callers' graphs name
+  bool own_capture = false;  // the graph cache is capturing
   unsigned ws_generation = 0;  // bumped whenever the workspace moves
   int graph_cache = 0;         // replay repeated identical single / mp calls
   // host-memory calls: device staging of three slots, the two copy streams

@@ -104,3 +104,42 @@ def test_graph_keeps_its_workspace(stream):
         stream.synchronize()
     for b, g in zip(small, graphs):
         b.check(g, 5)
+
+
+def test_stack_calls_in_a_capture(stream):
+    """LibShalom_dgemm_stack: the front-end buffer (72 bytes a product) grows in a
+    capture, and a graph keeps the one it names."""
+    import torch
+    m, n, k, many = 5, 4, 3, 30_000
+
+    def call(count):
+        g = torch.Generator(device="cuda").manual_seed(count)
+        A, B = (torch.rand(count * x, generator=g, device="cuda", dtype=torch.float64)
+                for x in (m * k, k * n))
+        C = torch.zeros(count * m * n, device="cuda", dtype=torch.float64)
+        offs = [torch.arange(count, device="cuda") * x for x in (m * k, k * n, m * n)]
+        ref = torch.bmm(A.view(count, m, k), B.view(count, k, n)).reshape(-1)
+        return C, ref, lambda: ls.dgemm_stack(A, B, C, *offs, count, m=m, n=n, k=k), (A, B, offs)
+
+    graphs = []
+    for count in (200, many):
+        C, ref, run, keep = call(count)
+        torch.cuda.synchronize()
+        if count == 200:
+            run()
+            torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            run()
+        graphs.append((C, ref, g, keep))
+    big = call(2 * many)  # outgrows both
+    torch.cuda.synchronize()
+    big[2]()
+    torch.cuda.synchronize()
+    for C, ref, g, _ in graphs:
+        C.zero_()
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        # both sides: k roundings of sums of k terms below 1
+        assert torch.max(torch.abs(C - ref)) <= 2 * k * k * 2.0 ** -53
