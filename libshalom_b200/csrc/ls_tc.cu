@@ -2067,7 +2067,9 @@ int tc_launch(TcProblem &p, int mode) {
     sa.M = p.M; sa.N = p.N; sa.K = p.K; sa.transb = p.transb;
     sa.alpha = p.alpha; sa.beta = p.beta;
     sa.tiles_n = (int)cdiv(p.N, SM_SMALL_TN);
-    const bool hold = p.K > SM_SMALL_CHUNK && p.beta != 0.0f;
+    // (C matrices that overlap hold no sums: each element is to be one product's)
+    const bool overlap = p.count > 1 && p.sC < (long)(p.M - 1) * p.ldc + p.N;
+    const bool hold = p.K > SM_SMALL_CHUNK && (p.beta != 0.0f || overlap);
     sa.tiles = (int)cdiv(p.M, hold ? SM_SUM_ROWS : SM_SMALL_TM) * sa.tiles_n;
     sa.n_items = (long)sa.tiles * p.count;
     sa.err = p.err;

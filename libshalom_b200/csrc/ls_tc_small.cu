@@ -28,8 +28,8 @@
 // bits.  C is updated once, after the last chunk: adding chunk after chunk into
 // a C that is large beside the product would round the product away (|C| =
 // 1,000, K = 2,048: normwise error 2.2e-7 against 3.7e-8).  Until then the sum
-// is kept in C itself by products that do not read C (beta = 0).  Products of
-// several chunks that do read it have a loop of their own (HOLD) that keeps the
+// is kept in C itself by products that do not read C (beta = 0) and have it to
+// themselves.  Other products of several chunks have a loop of their own (HOLD) that keeps the
 // sum in TMEM beside the accumulators, where there is room for tiles of up to 32
 // rows: as a branch of one loop it cost the others 8 % (registers and code), as a
 // launch of its own 8 us a call.
@@ -393,6 +393,10 @@ __global__ void __launch_bounds__(SM_THREADS, SM_PER_SM) k_tc_small(const TcSmal
                                        : pack2(c[w], c[w + 1]);
             unpack2(fma2(scale, d2, s2), v[w], v[w + 1]);
           }
+          if (UNIFORM && HOLD && last) {
+#pragma unroll
+            for (int w = 0; w < ER; ++w) v[w] *= alpha;
+          }
           if (HOLD && !last) {
             ptx::tmem_st8(acc + SM_SUM + r, v);
           } else if (how == 1) {
@@ -404,7 +408,7 @@ __global__ void __launch_bounds__(SM_THREADS, SM_PER_SM) k_tc_small(const TcSmal
               if (HOLD || first) {
 #pragma unroll
                 for (int w = 0; w < ER; ++w)
-                  v[w] = __fmaf_rn(beta, c[w], UNIFORM && HOLD ? alpha * v[w] : v[w]);
+                  v[w] = __fmaf_rn(beta, c[w], v[w]);
               } else if (UNIFORM && last) {
 #pragma unroll
                 for (int w = 0; w < ER; ++w) v[w] *= alpha;

@@ -113,3 +113,16 @@ def test_subnormal_c_is_kept():
         C = to_dev(C0)
         ls.sgemm_ex(0, 0, M, N, K, 1.0, A, max(K, 1), B, N, 1.0, C, N)
         assert np.array_equal(to_host(C), C0)
+
+
+@pytest.mark.parametrize("alpha", [1.0, 0.3])
+def test_products_on_one_c(alpha):
+    """Equal products that all name one C (strides 0): every element is the
+    product's, also while the others write it."""
+    ls.set_precision(ls.PREC_BF16X6)
+    for M, N, K in ((45, 37, 300), (130, 129, 1025)):
+        A, B = to_dev(orc.uniform_f32(1, M * K)), to_dev(orc.uniform_f32(2, K * N))
+        C = [to_dev(np.full(M * N, np.nan, np.float32)) for _ in range(2)]
+        ls.sgemm_batched_strided(0, M, N, K, alpha, A, 0, B, 0, 0.0, C[0], 0, 2000)
+        ls.sgemm_batched_strided(0, M, N, K, alpha, A, 0, B, 0, 0.0, C[1], 0, 1)
+        assert np.array_equal(to_host(C[0]), to_host(C[1]))
