@@ -241,6 +241,7 @@ static int gemm_common(int transa, int transb, T *C, const T *A, const T *B, lon
 // ---------------------------------------------------------------------------
 struct GraphKey {
   int kind, transa, transb, precision, tile_cfg, autotune, splitk, ways_m, ways_n, device;
+  int thread_cap, use_tma;
   const void *A, *B, *C;
   long M, N, K;
   cudaStream_t stream;
@@ -283,6 +284,7 @@ static int gemm_cached(int kind, int transa, int transb, T *C, const T *A, const
   key.kind = kind; key.transa = transa; key.transb = transb; key.precision = st.precision;
   key.tile_cfg = st.tile_cfg; key.autotune = st.autotune; key.splitk = st.splitk;
   key.ways_m = st.ways_m; key.ways_n = st.ways_n; key.device = st.device;
+  key.thread_cap = st.thread_cap; key.use_tma = st.use_tma;
   key.A = A; key.B = B; key.C = C; key.M = M; key.N = N; key.K = K; key.stream = st.stream;
   auto &cache = graph_cache();
   auto it = cache.find(key);
