@@ -36,7 +36,7 @@
 //
 // Measured on a B200: 50,000 products of 4..256 (log-uniform, one in five
 // adding to its predecessor's C) 1.14 ms, against 2.66 ms with k_tc_grouped
-// alone; 10,000 products of 45 x 37 x 51 96 us, against 465 us with
+// alone; 10,000 products of 45 x 37 x 51 94 us, against 465 us with
 // k_tc_sgemm.  Bound by instruction issue and latency (ncu, the mixed batch:
 // 55-60 % fewer warp instructions than k_tc_grouped, issue slots 47 % busy,
 // L1 55 %, DRAM 22 %, tensor pipe 16 %).  What did not help: eight warps per CTA
@@ -405,7 +405,9 @@ __global__ void __launch_bounds__(SM_THREADS, SM_PER_SM) k_tc_small(const TcSmal
               red_add_if(reinterpret_cast<float *>(pc + ldcB * w), v[w], w < nr);
           } else {
             if (how == 2) {
-              if (HOLD || first) {
+              // (C was read for beta; the two forms are one condition, each the
+              // faster code in its kernel: 45 x 37 x 51 93.5 us against 96.6)
+              if (UNIFORM ? last && beta != 0.0f : HOLD || first) {
 #pragma unroll
                 for (int w = 0; w < ER; ++w)
                   v[w] = __fmaf_rn(beta, c[w], v[w]);
